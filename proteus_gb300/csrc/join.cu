@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(kThreads)
 
 // Probe with fused aggregate over the bucketed table.  A probe visits its
 // home bucket and folds every slot whose key matches into the aggregate
-// without branching (a count of the matches and, for the specialised
-// aggregate lists, a select-and-sum of their values); it moves on to the
+// without branching (a count of the matches and a select-and-sum of their
+// values, for the two specialised aggregate lists); it moves on to the
 // next bucket only when the bucket is full and either has no match or the
 // build keys are not unique -- the rare case, taken out of line.  Each
 // thread handles kJbGroup probes at a time: their bucket loads (one 256-bit
@@ -267,26 +267,20 @@ __global__ void __launch_bounds__(kThreads)
 // payloads are loaded while they are in flight.  kPay: the values are build
 // payloads and build rows come from the row array.
 template <bool kVec, int kAgg, bool kPay>
-__global__ void __launch_bounds__(kThreads, kAgg == kAggGeneric ? 1 : GBJ_JB_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, GBJ_JB_MIN_BLOCKS)
     k_jb_probe_agg(const int32_t *__restrict__ keys, const int32_t *__restrict__ pay, uint64_t n,
                    const JBucket *__restrict__ bk, const int4 *__restrict__ rows, uint32_t bmask,
                    const int32_t *__restrict__ bpay, const uint32_t *__restrict__ meta,
                    const int32_t *__restrict__ side, gbj::AggSpec spec, int64_t *out) {
   __shared__ int64_t red[32 * GBJ_MAX_AGGS];
-  gbjd::Acc acc;  // the specialised accumulators fill it only at the end
-  if (kAgg == kAggGeneric) acc.init(spec);
+  static_assert(kAgg != kAggGeneric, "other aggregate lists: k_jb_probe_list");
   int64_t a_cnt = 0, a_sum = 0;
   const bool unique = meta[0] == 0;
   const uint32_t nside = meta[1];
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  // does the generic aggregate list read build rows? (payload tables keep them apart)
-  bool need_row = !kPay;
-  if (kPay && kAgg == kAggGeneric)
-    for (int j = 0; j < spec.n; ++j)
-      need_row |= spec.operand[j] == GBJ_VAL_BUILD_ROWID || spec.operand[j] == GBJ_VAL_ROWID_XOR;
   // folds the matching slots of bucket b (contents e) into the aggregate;
   // returns the number of matches
-  auto visit = [&](int32_t k, int32_t kf, int64_t pv, uint64_t prow, uint32_t b, const JBucket &e) -> uint32_t {
+  auto visit = [&](int32_t kf, int64_t pv, uint64_t prow, uint32_t b, const JBucket &e) -> uint32_t {
     const bool m0 = e.k.x == kf, m1 = e.k.y == kf, m2 = e.k.z == kf, m3 = e.k.w == kf;
     const uint32_t c = (uint32_t)m0 + (uint32_t)m1 + (uint32_t)m2 + (uint32_t)m3;
     if (kAgg == kAggCountProduct) {
@@ -299,58 +293,44 @@ __global__ void __launch_bounds__(kThreads, kAgg == kAggGeneric ? 1 : GBJ_JB_MIN
       a_sum += (m0 ? ((int64_t)(e.x.x - 1) ^ pr) : 0) + (m1 ? ((int64_t)(e.x.y - 1) ^ pr) : 0) +
                (m2 ? ((int64_t)(e.x.z - 1) ^ pr) : 0) + (m3 ? ((int64_t)(e.x.w - 1) ^ pr) : 0);
     } else if (c) {
-      const bool rows_needed = kAgg == kAggCountXor || need_row;
-      const int4 rw = kPay && rows_needed ? __ldg(&rows[b]) : e.x;
+      const int4 rw = kPay ? __ldg(&rows[b]) : e.x;
       uint32_t hits = (uint32_t)m0 | ((uint32_t)m1 << 1) | ((uint32_t)m2 << 2) | ((uint32_t)m3 << 3);
       while (hits) {
         const uint32_t idx = __ffs(hits) - 1;
-        const int64_t bv = kPay ? lane4(e.x, idx) : 0;
-        const int64_t brow = (kPay && !rows_needed) ? 0 : lane4(rw, idx) - 1;
-        if (kAgg == kAggCountXor) {
-          a_cnt += 1;
-          a_sum += brow ^ (int64_t)prow;
-        } else {
-          acc.update(spec, k, bv, pv, brow, prow);
-        }
+        a_cnt += 1;
+        a_sum += (int64_t)(lane4(rw, idx) - 1) ^ (int64_t)prow;
         hits &= hits - 1;
       }
     }
     return c;
   };
   // the buckets after a full home bucket (out of line, rare)
-  auto walk = [&](int32_t k, int32_t kf, int64_t pv, uint64_t prow, uint32_t b, uint32_t matched) {
+  auto walk = [&](int32_t kf, int64_t pv, uint64_t prow, uint32_t b, uint32_t matched) {
     for (uint32_t step = 1; step <= bmask; ++step) {
       b = (b + 1) & bmask;
       const JBucket e = ld_bucket(&bk[b]);
-      matched += visit(k, kf, pv, prow, b, e);
+      matched += visit(kf, pv, prow, b, e);
       if (room4(e.k) || (unique && matched)) return;
     }
   };
   // a probe key INT32_MIN meets the side list
-  auto side_probe = [&](int32_t k, int64_t pv, uint64_t prow) {
+  auto side_probe = [&](int64_t pv, uint64_t prow) {
     for (uint32_t s = 0; s < nside; ++s) {
       const int32_t r = side[s];
-      const int64_t bv = kPay ? (int64_t)bpay[r] : 0;
-      if (kAgg == kAggCountProduct) {
-        a_cnt += 1;
-        a_sum += bv * pv;
-      } else if (kAgg == kAggCountXor) {
-        a_cnt += 1;
-        a_sum += (int64_t)r ^ (int64_t)prow;
-      } else {
-        acc.update(spec, k, bv, pv, r, prow);
-      }
+      a_cnt += 1;
+      if (kAgg == kAggCountProduct) a_sum += (kPay ? (int64_t)bpay[r] : 0) * pv;
+      else a_sum += (int64_t)r ^ (int64_t)prow;
       if (unique) break;
     }
   };
   auto finish = [&](int32_t k, int64_t pv, uint64_t prow, uint32_t b, const JBucket &e) {
     const int32_t kf = k ^ kKeyFlip;
     if (kf == 0) {
-      side_probe(k, pv, prow);
+      side_probe(pv, prow);
       return;
     }
-    const uint32_t c = visit(k, kf, pv, prow, b, e);
-    if (!room4(e.k) && !(unique && c)) walk(k, kf, pv, prow, b, c);
+    const uint32_t c = visit(kf, pv, prow, b, e);
+    if (!room4(e.k) && !(unique && c)) walk(kf, pv, prow, b, c);
   };
   uint64_t done = 0;
   if (kVec) {
@@ -393,11 +373,10 @@ __global__ void __launch_bounds__(kThreads, kAgg == kAggGeneric ? 1 : GBJ_JB_MIN
     const uint32_t b = gbjd::fmix32((uint32_t)k) & bmask;
     finish(k, pay ? pay[i] : 0, i, b, ld_bucket(&bk[b]));
   }
-  if (kAgg != kAggGeneric) {
-    acc.init(spec);
-    acc.v[0] = a_cnt;
-    acc.v[1] = a_sum;
-  }
+  gbjd::Acc acc;
+  acc.init(spec);
+  acc.v[0] = a_cnt;
+  acc.v[1] = a_sum;
   gbjd::block_flush(spec, acc, red, out);
 }
 
@@ -530,76 +509,245 @@ __global__ void __launch_bounds__(kThreads)
   if (dup) meta[0] = 1;
 }
 
-// Probe with fused aggregate over the int64-key table: four probes per
-// thread, their bucket loads issued together; a probe moves past its home
-// bucket only when it is full and (for unique build keys) has no match.
-__global__ void __launch_bounds__(kThreads)
-    k_jb64_probe_agg(const int64_t *__restrict__ keys, const int32_t *__restrict__ pay, uint64_t n,
-                     const JBucket64 *__restrict__ bk, uint64_t bmask, const int32_t *__restrict__ bpay,
-                     const uint32_t *__restrict__ meta, const int32_t *__restrict__ side, gbj::AggSpec spec,
-                     int64_t *out) {
+// ------------------------------------------------ probe with any aggregate list
+// The two table layouts as k_jb_probe_list reads them.
+struct JTable {
+  const void *bk;
+  const int4 *rows;
+  uint32_t bmask;  // buckets - 1
+  const int32_t *bpay;
+  const uint32_t *meta;
+  const int32_t *side;
+};
+
+template <bool kPay>
+struct JLayout32 {
+  using Key = int32_t;
+  using Word = int32_t;  // the key as stored; 0 is the empty slot
+  using Bucket = JBucket;
+  static __device__ __forceinline__ Word word(Key k) { return k ^ kKeyFlip; }
+  static __device__ __forceinline__ uint32_t home(Key k, uint32_t m) { return gbjd::fmix32((uint32_t)k) & m; }
+  static __device__ __forceinline__ Bucket load(const JTable &t, uint32_t b) {
+    return ld_bucket(static_cast<const JBucket *>(t.bk) + b);
+  }
+  static __device__ __forceinline__ uint32_t hits(const Bucket &e, Word w) { return hits4(e.k, w); }
+  static __device__ __forceinline__ bool room(const Bucket &e) { return room4(e.k); }
+  static __device__ __forceinline__ int32_t value(const Bucket &e, uint32_t i) { return kPay ? lane4(e.x, i) : 0; }
+  static __device__ __forceinline__ int32_t row(const JTable &t, const Bucket &e, uint32_t b, uint32_t i) {
+    return (kPay ? __ldg(reinterpret_cast<const int32_t *>(t.rows + b) + i) : lane4(e.x, i)) - 1;
+  }
+};
+
+struct JLayout64 {
+  using Key = int64_t;
+  using Word = unsigned long long;
+  using Bucket = JBucket64;
+  static __device__ __forceinline__ Word word(Key k) { return (unsigned long long)k ^ kFlip64; }
+  static __device__ __forceinline__ uint32_t home(Key k, uint32_t m) { return (uint32_t)fmix64((uint64_t)k) & m; }
+  static __device__ __forceinline__ Bucket load(const JTable &t, uint32_t b) {
+    return ld_bucket64(static_cast<const JBucket64 *>(t.bk) + b);
+  }
+  static __device__ __forceinline__ uint32_t hits(const Bucket &e, Word w) {
+    return (uint32_t)(e.k[0] == w) | ((uint32_t)(e.k[1] == w) << 1);
+  }
+  static __device__ __forceinline__ bool room(const Bucket &e) { return (e.k[0] == 0) | (e.k[1] == 0); }
+  static __device__ __forceinline__ int32_t value(const Bucket &e, uint32_t i) { return i ? e.x[1] : e.x[0]; }
+  static __device__ __forceinline__ int32_t row(const JTable &, const Bucket &e, uint32_t, uint32_t i) {
+    return (i ? e.r[1] : e.r[0]) - 1;
+  }
+};
+
+constexpr int kListThreads = 256;
+// CTAs per SM of k_jb_probe_list.  Measured on the case below with unique
+// keys: 3 (80 registers) 234 us, 4 (64, spills) 268, 5 (48, spills) 452.
+constexpr int kListCtas = 3;
+constexpr int kListWarps = kListThreads / 32;
+
+// A warp's queues, both rings: matches on their way to the accumulators, and
+// probes that go on past their home bucket (the last bucket looked at, and
+// how many are left; for the lowest key, which has no bucket, the next side
+// entry).
+template <typename Key>
+struct ListQueue {
+  Key mkey[64];
+  uint64_t mprow[64];
+  int32_t mbv[64], mpv[64], mbr[64];
+  Key wkey[64];
+  uint64_t wprow[64];
+  int32_t wpv[64];
+  uint32_t wb[64], wleft[64];
+};
+
+// Probe with an aggregate list that has no specialised kernel, and every
+// list over int64 keys.  One probe per lane at a time: the next one's bucket
+// is loaded while this one's is looked at, and its key one step earlier.
+//
+// What bounds it is issue.  The accumulator update takes some 20 instructions
+// per aggregate, and matches are few lanes of a warp at a time when they are
+// applied where they are found; inlined at each of the places where a match
+// can turn up it also overran the instruction cache (31 of 38 stalled warps
+// per issue waited for instructions, 8.4 active lanes).  So a match goes to
+// the warp's ring of 64, and 32 of them are applied at once by all lanes;
+// probes whose home bucket is full go to a second ring, from which 32 at a
+// time look at their next bucket and go back if that does not end them.
+// Measured on GB300, 1.5 M int64 build rows (two per key), 20 M probes, COUNT
+// + SUM + MIN + MAX: 8.21 ms before, 0.54 ms now (one row per key: 4.54 -> 0.23
+// ms; the same over int32 keys: 0.90 -> 0.22 ms).
+template <typename L, int kMaxA>
+__global__ void __launch_bounds__(kListThreads, kListCtas)
+    k_jb_probe_list(const typename L::Key *__restrict__ keys, const int32_t *__restrict__ pay, uint64_t n,
+                    JTable t, gbj::AggSpec spec, int64_t *out) {
+  using Key = typename L::Key;
+  using Bucket = typename L::Bucket;
   __shared__ int64_t red[32 * GBJ_MAX_AGGS];
+  __shared__ ListQueue<Key> s_q[kListWarps];
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  ListQueue<Key> &q = s_q[threadIdx.x >> 5];
+  const bool unique = t.meta[0] == 0;
+  const uint32_t nside = t.meta[1];
+  bool need_row = false;
+#pragma unroll
+  for (int j = 0; j < kMaxA; ++j)
+    if (j < spec.n)
+      need_row |= spec.operand[j] == GBJ_VAL_BUILD_ROWID || spec.operand[j] == GBJ_VAL_ROWID_XOR;
+  int64_t v[kMaxA];
+#pragma unroll
+  for (int j = 0; j < kMaxA; ++j) v[j] = j < spec.n ? gbjd::agg_identity(spec.op[j]) : 0;
+
+  uint32_t mn = 0, mh = 0;  // the ring's length and head (warp-uniform)
+  // applies the first `c` (<= 32) matches of the ring
+  auto apply = [&](uint32_t c) {
+    __syncwarp();
+    if ((uint32_t)lane < c) {
+      const uint32_t p = (mh + lane) & 63u;
+      const int32_t bv = q.mbv[p], pv = q.mpv[p], br = q.mbr[p];
+      const int64_t pr = (int64_t)q.mprow[p];
+#pragma unroll
+      for (int j = 0; j < kMaxA; ++j) {
+        if (j < spec.n) {  // the list is the same for all lanes: uniform branches
+          const int o = spec.operand[j], op = spec.op[j];
+          int64_t x;
+          if (o <= GBJ_VAL_PROBE) x = o == GBJ_VAL_BUILD ? bv : o == GBJ_VAL_PROBE ? pv : 1;
+          else if (o == GBJ_VAL_PRODUCT) x = (int64_t)bv * pv;
+          else if (o == GBJ_VAL_BUILD_ROWID) x = br;
+          else if (o == GBJ_VAL_PROBE_ROWID) x = pr;
+          else if (o == GBJ_VAL_ROWID_XOR) x = (int64_t)br ^ pr;
+          else x = (int64_t)q.mkey[p];
+          if (op == GBJ_AGG_COUNT) v[j] += 1;
+          else if (op == GBJ_AGG_SUM) v[j] += x;
+          else if (op == GBJ_AGG_MIN) v[j] = x < v[j] ? x : v[j];
+          else if (op == GBJ_AGG_MAX) v[j] = x > v[j] ? x : v[j];
+          else if (op == GBJ_AGG_OR) v[j] |= (int64_t)(x != 0);
+          else v[j] &= (int64_t)(x != 0);
+        }
+      }
+    }
+    __syncwarp();
+    mh = (mh + c) & 63u;
+    mn -= c;
+  };
+  // every match of a bucket (or side row srow >= 0) into the ring; all lanes call it
+  auto push = [&](uint32_t hits, Key k, int32_t pv, uint64_t prow, uint32_t b, const Bucket &e, int32_t srow) {
+    for (;;) {
+      const unsigned bal = __ballot_sync(0xffffffffu, hits != 0);
+      if (!bal) break;
+      if (hits) {
+        const uint32_t i = __ffs(hits) - 1;
+        const uint32_t p = (mh + mn + __popc(bal & lt)) & 63u;
+        q.mkey[p] = k;
+        q.mprow[p] = prow;
+        q.mpv[p] = pv;
+        q.mbv[p] = srow < 0 ? L::value(e, i) : t.bpay ? __ldg(t.bpay + srow) : 0;
+        q.mbr[p] = srow >= 0 ? srow : need_row ? L::row(t, e, b, i) : 0;
+        hits = unique ? 0u : hits & (hits - 1);
+      }
+      mn += __popc(bal);
+      if (mn >= 32) apply(32);
+    }
+  };
+  uint32_t wn = 0, wh = 0;  // the second ring's length and head
+  auto queue_walk = [&](bool go_on, Key k, int32_t pv, uint64_t prow, uint32_t b, uint32_t left) {
+    const unsigned bal = __ballot_sync(0xffffffffu, go_on);
+    if (go_on) {
+      const uint32_t p = (wh + wn + __popc(bal & lt)) & 63u;
+      q.wkey[p] = k;
+      q.wprow[p] = prow;
+      q.wpv[p] = pv;
+      q.wb[p] = b;
+      q.wleft[p] = left;
+    }
+    wn += __popc(bal);
+  };
+  // one bucket (or side entry) further for the first `c` (<= 32) of them
+  auto walk = [&](uint32_t c) {
+    __syncwarp();
+    const bool active = (uint32_t)lane < c;
+    const uint32_t p = (wh + lane) & 63u;
+    const Key k = active ? q.wkey[p] : 0;
+    const uint64_t prow = active ? q.wprow[p] : 0;
+    const int32_t pv = active ? q.wpv[p] : 0;
+    uint32_t b = active ? q.wb[p] : 0;
+    const uint32_t left = active ? q.wleft[p] - 1 : 0;
+    __syncwarp();  // read before any of them is written again
+    wh = (wh + c) & 63u;
+    wn -= c;
+    uint32_t hits = 0;
+    int32_t srow = -1;
+    Bucket e{};
+    bool go_on = false;
+    if (active) {
+      if (L::word(k) == 0) {
+        srow = __ldg(t.side + b);
+        ++b;
+        hits = 1;
+        go_on = left != 0 && !unique;
+      } else {
+        b = (b + 1) & t.bmask;
+        e = L::load(t, b);
+        hits = L::hits(e, L::word(k));
+        go_on = left != 0 && !L::room(e) && !(unique && hits);
+      }
+    }
+    push(hits, k, pv, prow, b, e, srow);
+    queue_walk(go_on, k, pv, prow, b, left);
+  };
+
+  const uint64_t wstep = (uint64_t)gridDim.x * kListThreads;
+  const uint64_t first = blockIdx.x * (uint64_t)kListThreads + (threadIdx.x & ~31u);  // of the warp
+  auto load_key = [&](uint64_t i, Key &k, int32_t &p) {
+    k = i < n ? __ldcs(keys + i) : 0;
+    p = pay && i < n ? __ldcs(pay + i) : 0;
+  };
+  Key k0, k1;
+  int32_t p0, p1;
+  load_key(first + lane, k0, p0);
+  uint32_t b0 = L::home(k0, t.bmask);
+  Bucket e0 = L::load(t, b0);
+  load_key(first + wstep + lane, k1, p1);
+  for (uint64_t base = first; base < n; base += wstep) {
+    const Key k = k0;
+    const int32_t pv = p0;
+    const uint32_t b = b0;
+    const Bucket e = e0;
+    k0 = k1;
+    p0 = p1;
+    b0 = L::home(k0, t.bmask);
+    e0 = L::load(t, b0);
+    load_key(base + 2 * wstep + lane, k1, p1);
+    const uint64_t i = base + lane;
+    const bool valid = i < n, to_side = L::word(k) == 0;  // the lowest key is in the side list
+    const uint32_t hits = valid && !to_side ? L::hits(e, L::word(k)) : 0u;
+    push(hits, k, pv, i, b, e, -1);
+    const bool go_on = valid && (to_side ? nside != 0 : t.bmask != 0 && !L::room(e) && !(unique && hits));
+    queue_walk(go_on, k, pv, i, to_side ? 0u : b, to_side ? nside : t.bmask);
+    while (wn >= 32) walk(32);
+  }
+  while (wn) walk(wn < 32 ? wn : 32);
+  while (mn) apply(mn < 32 ? mn : 32);
   gbjd::Acc acc;
-  acc.init(spec);
-  const bool unique = meta[0] == 0;
-  const uint32_t nside = meta[1];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  auto visit = [&](int64_t k, unsigned long long kf, int64_t pv, uint64_t prow, const JBucket64 &e) -> uint32_t {
-    uint32_t c = 0;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      if (e.k[j] == kf) {
-        acc.update(spec, k, e.x[j], pv, (int64_t)e.r[j] - 1, (int64_t)prow);
-        ++c;
-      }
-    }
-    return c;
-  };
-  auto room = [](const JBucket64 &e) { return e.k[0] == 0 || e.k[1] == 0; };
-  auto finish = [&](int64_t k, int64_t pv, uint64_t prow, uint64_t b, const JBucket64 &e0) {
-    const unsigned long long kf = (unsigned long long)k ^ kFlip64;
-    if (kf == 0) {  // INT64_MIN meets the side list
-      for (uint32_t s = 0; s < nside; ++s) {
-        const int32_t r = side[s];
-        acc.update(spec, k, bpay ? (int64_t)bpay[r] : 0, pv, r, (int64_t)prow);
-        if (unique) break;
-      }
-      return;
-    }
-    uint32_t matched = visit(k, kf, pv, prow, e0);
-    if (room(e0) || (unique && matched)) return;
-    for (uint64_t step = 1; step <= bmask; ++step) {
-      b = (b + 1) & bmask;
-      const JBucket64 e = ld_bucket64(&bk[b]);
-      matched += visit(k, kf, pv, prow, e);
-      if (room(e) || (unique && matched)) return;
-    }
-  };
-  constexpr int G = 4;
-  const uint64_t ng = n / G;
-  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < ng; q += stride) {
-    int64_t kk[G];
-    int64_t pp[G];
-    uint64_t b[G];
-    JBucket64 e[G];
-#pragma unroll
-    for (int j = 0; j < G; ++j) {
-      kk[j] = __ldcs(keys + q * G + j);
-      pp[j] = pay ? __ldcs(pay + q * G + j) : 0;
-    }
-#pragma unroll
-    for (int j = 0; j < G; ++j) {
-      b[j] = fmix64((uint64_t)kk[j]) & bmask;
-      e[j] = ld_bucket64(&bk[b[j]]);
-    }
-#pragma unroll
-    for (int j = 0; j < G; ++j) finish(kk[j], pp[j], q * G + j, b[j], e[j]);
-  }
-  for (uint64_t i = ng * G + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int64_t k = keys[i];
-    const uint64_t b = fmix64((uint64_t)k) & bmask;
-    finish(k, pay ? pay[i] : 0, i, b, ld_bucket64(&bk[b]));
-  }
+  for (int j = 0; j < GBJ_MAX_AGGS; ++j) acc.v[j] = j < kMaxA ? v[j < kMaxA ? j : 0] : 0;
   gbjd::block_flush(spec, acc, red, out);
 }
 
@@ -724,6 +872,20 @@ void launch_probe(int sm_count, const int32_t *keys, const int32_t *pay, uint64_
 #undef GBJ_PROBE
 }
 
+// Any other list, and every list over int64 keys: kernels for up to four and
+// up to eight aggregates (the accumulators are registers).
+template <typename L>
+void launch_jb_list(int sm_count, const gbj_table *t, uint64_t nbk, const typename L::Key *keys, const int32_t *pay,
+                    uint64_t n, const gbj::AggSpec &spec, int64_t *out, cudaStream_t s) {
+  const JTable jt{t->slots, t->rows, (uint32_t)(nbk - 1), t->payload, t->meta, t->side};
+  if (spec.n <= 4)
+    k_jb_probe_list<L, 4><<<grid_for_sms(sm_count, n, kListThreads, kListCtas), kListThreads, 0, s>>>(keys, pay, n, jt, spec,
+                                                                                            out);
+  else
+    k_jb_probe_list<L, 8><<<grid_for_sms(sm_count, n, kListThreads, kListCtas), kListThreads, 0, s>>>(keys, pay, n, jt, spec,
+                                                                                            out);
+}
+
 // Probe kernel over a bucketed table: 16-byte probe loads when both probe
 // columns are aligned, the specialised accumulators, the table's layout.
 template <bool kPay>
@@ -731,24 +893,25 @@ void launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, co
                        const gbj::AggSpec &spec, int64_t *out, cudaStream_t s) {
   const bool vec = ((uintptr_t)keys % 16 == 0) && (!pay || (uintptr_t)pay % 16 == 0);
   const bool two = spec.n == 2 && spec.op[0] == GBJ_AGG_COUNT && spec.op[1] == GBJ_AGG_SUM;
-  const int agg = two && spec.operand[1] == GBJ_VAL_ROWID_XOR ? kAggCountXor
-                  : two && spec.operand[1] == GBJ_VAL_PRODUCT ? kAggCountProduct
-                                                              : kAggGeneric;
+  const bool is_xor = two && spec.operand[1] == GBJ_VAL_ROWID_XOR;
   const JBucket *bk = static_cast<const JBucket *>(t->slots);
-  const uint32_t bmask = (uint32_t)((t->mask + 1) / 4 - 1);
+  const uint64_t nbk = (t->mask + 1) / 4;
+  const uint32_t bmask = (uint32_t)(nbk - 1);
+  if (!is_xor && !(two && spec.operand[1] == GBJ_VAL_PRODUCT)) {
+    launch_jb_list<JLayout32<kPay>>(sm_count, t, nbk, keys, pay, n, spec, out, s);
+    return;
+  }
   const int gv = grid_for_sms(sm_count, (n + kJbGroup - 1) / kJbGroup, kThreads, 2);
   const int gs = grid_for_sms(sm_count, n, kThreads);
 #define GBJ_JB_PROBE(V, A)                                                                               \
   k_jb_probe_agg<V, A, kPay><<<V ? gv : gs, kThreads, 0, s>>>(keys, pay, n, bk, t->rows, bmask, t->payload, \
                                                               t->meta, t->side, spec, out)
   if (vec) {
-    if (agg == kAggCountXor) GBJ_JB_PROBE(true, kAggCountXor);
-    else if (agg == kAggCountProduct) GBJ_JB_PROBE(true, kAggCountProduct);
-    else GBJ_JB_PROBE(true, kAggGeneric);
+    if (is_xor) GBJ_JB_PROBE(true, kAggCountXor);
+    else GBJ_JB_PROBE(true, kAggCountProduct);
   } else {
-    if (agg == kAggCountXor) GBJ_JB_PROBE(false, kAggCountXor);
-    else if (agg == kAggCountProduct) GBJ_JB_PROBE(false, kAggCountProduct);
-    else GBJ_JB_PROBE(false, kAggGeneric);
+    if (is_xor) GBJ_JB_PROBE(false, kAggCountXor);
+    else GBJ_JB_PROBE(false, kAggCountProduct);
   }
 #undef GBJ_JB_PROBE
 }
@@ -1019,10 +1182,8 @@ int gbj_join_probe_agg_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_ke
   prof_mark(ctx, s);
   GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
   if (n == 0) return GBJ_OK;
-  k_jb64_probe_agg<<<grid_for(ctx, (n + 3) / 4, kThreads, 2), kThreads, 0, s>>>(
-      d_keys, d_payload, n, static_cast<const JBucket64 *>(t->slots), (t->mask + 1) / 2 - 1, t->payload, t->meta,
-      t->side, spec, d_out);
-  return after_launch(ctx, "k_jb64_probe_agg", s);
+  launch_jb_list<JLayout64>(ctx->sm_count, t, (t->mask + 1) / 2, d_keys, d_payload, n, spec, d_out, s);
+  return after_launch(ctx, "k_jb_probe_list", s);
 }
 
 int gbj_join_probe_pairs_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_keys,
