@@ -1,0 +1,43 @@
+"""Grouping int64 keys in the global table: row counts around a warp and its
+ring, groups whose home slots collide, INT64_MIN, every value form, and the
+number of groups a table takes, against the oracle."""
+import numpy as np
+import pytest
+
+from gpu_util import dev, host
+from proteus_gb300 import abi
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("with_vals", [True, False])
+@pytest.mark.parametrize("n,groups,expected", [(1, 1, 0), (33, 20, 4000), (65, 65, 0), (4097, 4000, 4000),
+                                               (100_003, 60_000, 60_000), (300_001, 3000, 2500),
+                                               (200_000, 7, 70_000)])
+def test_global_table(ctx, oracle, n, groups, expected, with_vals):
+    rng = np.random.default_rng(n)
+    keys = rng.integers(-(1 << 62), 1 << 62, groups)[rng.integers(0, groups, n)]
+    keys[::97] = np.iinfo(np.int64).min
+    vals = rng.integers(-(1 << 63), (1 << 63) - 1, n) if with_vals else None
+    got = ctx.nest_i64(dev(keys), dev(vals) if with_vals else None, n + 1, expected_groups=expected)
+    ctx.sync()
+    m = int(host(got[5])[0])
+    order = np.argsort(host(got[0])[:m])
+    for g, e in zip(got[:5], oracle.nest_i64(keys, vals)):
+        assert (host(g)[:m][order] == e).all()
+
+
+@pytest.mark.parametrize("extra,ok", [(0, True), (1, False)])
+@pytest.mark.parametrize("with_min", [False, True])
+def test_groups_a_table_takes(ctx, extra, ok, with_min):
+    """expected_groups = 2500 sizes it for 8192 groups, whatever its slots."""
+    keys = np.arange(8192 + extra, dtype=np.int64) * 3
+    keys = np.concatenate([keys, keys, [np.iinfo(np.int64).min] * with_min]).astype(np.int64)
+    got = ctx.nest_i64(dev(keys), dev(keys), 10_000, expected_groups=2500)
+    if ok:
+        ctx.sync()
+        assert int(host(got[5])[0]) == 8192 + with_min
+    else:
+        with pytest.raises(abi.GbjError) as e:
+            ctx.sync()
+        assert e.value.code == abi.ERR_CAPACITY
