@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kThreads)
       const bool here = e[u].key == ((unsigned long long)k[u] ^ kFlip64);
       add(ok[u] && here ? (int64_t)h[u] : -1, v[u], e[u]);
       push(ok[u] && !here, k[u], v[u], e[u].key == 0 ? h[u] : (h[u] + 1) & t.mask, t.mask);
-      if (qn >= 32) step(32);
+      while (qn >= 32) step(32);
     }
   }
   while (qn) step(qn < 32 ? qn : 32);

@@ -41,3 +41,25 @@ def test_groups_a_table_takes(ctx, extra, ok, with_min):
         with pytest.raises(abi.GbjError) as e:
             ctx.sync()
         assert e.value.code == abi.ERR_CAPACITY
+
+
+def test_long_chains(ctx, oracle):
+    """Keys of one home slot: every row is looked up again and again, so that
+    the warps' rings are full while new rows arrive."""
+    rng = np.random.default_rng(9)
+    cand = rng.integers(-(1 << 62), 1 << 62, 1 << 21)
+    h = cand.astype(np.uint64)
+    for factor in (0xFF51AFD7ED558CCD, 0xC4CEB9FE1A85EC53):  # the table's placement hash
+        h ^= h >> np.uint64(33)
+        h *= np.uint64(factor)
+    h ^= h >> np.uint64(33)
+    chain = cand[(h & np.uint64(32767)) == 0]
+    assert len(chain) > 40
+    keys = chain[rng.integers(0, len(chain), 2_000_000)]  # several rounds of every warp
+    vals = rng.integers(-1000, 1000, len(keys))
+    got = ctx.nest_i64(dev(keys), dev(vals), 1000, expected_groups=2500)
+    ctx.sync()
+    m = int(host(got[5])[0])
+    order = np.argsort(host(got[0])[:m])
+    for g, e in zip(got[:5], oracle.nest_i64(keys, vals)):
+        assert (host(g)[:m][order] == e).all()
