@@ -625,22 +625,8 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
       const int64_t pr = (int64_t)q.mprow[p];
 #pragma unroll
       for (int j = 0; j < kMaxA; ++j) {
-        if (j < spec.n) {  // the list is the same for all lanes: uniform branches
-          const int o = spec.operand[j], op = spec.op[j];
-          int64_t x;
-          if (o <= GBJ_VAL_PROBE) x = o == GBJ_VAL_BUILD ? bv : o == GBJ_VAL_PROBE ? pv : 1;
-          else if (o == GBJ_VAL_PRODUCT) x = (int64_t)bv * pv;
-          else if (o == GBJ_VAL_BUILD_ROWID) x = br;
-          else if (o == GBJ_VAL_PROBE_ROWID) x = pr;
-          else if (o == GBJ_VAL_ROWID_XOR) x = (int64_t)br ^ pr;
-          else x = (int64_t)q.mkey[p];
-          if (op == GBJ_AGG_COUNT) v[j] += 1;
-          else if (op == GBJ_AGG_SUM) v[j] += x;
-          else if (op == GBJ_AGG_MIN) v[j] = x < v[j] ? x : v[j];
-          else if (op == GBJ_AGG_MAX) v[j] = x > v[j] ? x : v[j];
-          else if (op == GBJ_AGG_OR) v[j] |= (int64_t)(x != 0);
-          else v[j] &= (int64_t)(x != 0);
-        }
+        if (j < spec.n)
+          gbjd::agg_step(v[j], spec.op[j], spec.operand[j], (int64_t)q.mkey[p], bv, pv, br, pr);
       }
     }
     __syncwarp();
