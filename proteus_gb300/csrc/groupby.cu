@@ -527,12 +527,13 @@ __global__ void k_groupby_emit(GTable g, Out o, uint32_t *status) {
   }
 }
 
-__global__ void k_groupby_items(const uint64_t *__restrict__ poff, uint32_t P, uint64_t w,
-                                uint64_t *__restrict__ items) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  const uint64_t m = poff[p + 1] - poff[p];
-  items[p] = (m + w - 1) / w;
+// Work items of w rows per partition, as offsets, and the item counter.
+__global__ void __launch_bounds__(1024)
+    k_groupby_plan(const uint64_t *__restrict__ poff, uint32_t P, uint64_t w, uint64_t *__restrict__ items,
+                   unsigned long long *ctr) {
+  __shared__ uint64_t s_scan[32];
+  if (threadIdx.x == 0) *ctr = 0;
+  gbjd::cta_offsets(P, [&](uint32_t p) { return (poff[p + 1] - poff[p] + w - 1) / w; }, items, s_scan);
 }
 
 }  // namespace
@@ -589,7 +590,6 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
         reinterpret_cast<unsigned long long *>(d_n_groups)};
   unsigned long long *ctr;
   GBJ_TRY(scratch.get(1, &ctr));
-  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
 
   uint32_t tslots_arg = kSlots, rlog_arg = 0;
   // as many accumulator columns (up to 32) as the table budget allows
@@ -610,6 +610,7 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
   };
 
   if (strategy == 1) {
+    GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
     // raw input in items of w rows; level 1 persists for the CTA's lifetime
     const uint64_t w = std::max<uint64_t>(1u << 16, (n + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8));
     const uint64_t wq = (w + 3) / 4 * 4;
@@ -641,9 +642,8 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
     GBJ_TRY(scratch.get(P + 1, &items));
     GBJ_TRY(partition_tuples(ctx, d_keys, d_values, n, GBJ_DIGIT_HASH, 0, bits, pairs, nullptr,
                              nullptr, poff, s));
-    k_groupby_items<<<(P + 255) / 256, 256, 0, s>>>(poff, P, w, items);
-    GBJ_TRY(after_launch(ctx, "k_groupby_items", s));
-    GBJ_TRY(scan_u64(ctx, items, items, P, s));
+    k_groupby_plan<<<1, 1024, 0, s>>>(poff, P, w, items, ctr);
+    GBJ_TRY(after_launch(ctx, "k_groupby_plan", s));
     GBJ_TRY(launch(k_groupby<true, false>, (int)tslots_arg, pairs, w, poff, items, P));
   }
   const uint64_t emit_threads = 256;

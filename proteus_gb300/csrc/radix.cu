@@ -83,13 +83,32 @@ __device__ __forceinline__ uint32_t digit_of(int32_t key, int shift, uint32_t ma
   return (v >> shift) & mask;
 }
 
+// What the passes need, written by the histogram's last CTA: offsets of the
+// P partitions and the output cursors; with two passes also the pass-1
+// buckets' (partition >> bits2) offsets, cursors and the prefix of their
+// tiles of `tile2` tuples.
+struct PartPlan {
+  uint64_t *off;       // [P + 1]
+  uint32_t *cursor;    // [P]
+  uint64_t *boff;      // [B1 + 1], null: one pass
+  uint32_t *bcursor;   // [B1]
+  uint64_t *btiles;    // [B1 + 1]
+  int bits2;
+  uint32_t tile2;
+};
+
 // Global histogram of partition ids (shared-memory counts, one global
-// atomic per non-empty bin and CTA).
+// atomic per non-empty bin and CTA), and the plan of the passes: the last
+// CTA to finish works it out, which takes the place of nine launches (a
+// multi-level scan, the cursors, the buckets' tiles and their scan).
+// ghist[P] counts the CTAs that are done.
 template <int kDigit>
 __global__ void __launch_bounds__(1024)
     k_pid_hist(const int32_t *__restrict__ keys, uint64_t n, int shift, uint32_t pmask,
-               uint32_t *__restrict__ ghist) {
+               uint32_t *ghist, PartPlan plan) {
   extern __shared__ uint32_t sh[];
+  __shared__ uint64_t s_scan[32];
+  __shared__ bool s_last;
   const uint32_t P = pmask + 1;
   for (uint32_t p = threadIdx.x; p < P; p += blockDim.x) sh[p] = 0;
   __syncthreads();
@@ -127,6 +146,25 @@ __global__ void __launch_bounds__(1024)
   __syncthreads();
   for (uint32_t p = threadIdx.x; p < P; p += blockDim.x)
     if (sh[p]) atomicAdd(&ghist[p], sh[p]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&ghist[P], 1u) + 1 == gridDim.x;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  gbjd::cta_offsets(P, [&](uint32_t p) -> uint64_t { return __ldcg(ghist + p); }, plan.off, s_scan);
+  __syncthreads();
+  for (uint32_t p = threadIdx.x; p < P; p += 1024) plan.cursor[p] = (uint32_t)plan.off[p];
+  if (!plan.boff) return;
+  const uint32_t B1 = P >> plan.bits2;
+  for (uint32_t b = threadIdx.x; b <= B1; b += 1024) {
+    const uint64_t o = plan.off[b << plan.bits2];
+    plan.boff[b] = o;
+    if (b < B1) plan.bcursor[b] = (uint32_t)o;
+  }
+  __syncthreads();
+  gbjd::cta_offsets(B1, [&](uint32_t b) { return (plan.boff[b + 1] - plan.boff[b] + plan.tile2 - 1) / plan.tile2; },
+                    plan.btiles, s_scan);
 }
 
 template <int kSh>
@@ -380,39 +418,21 @@ __global__ void __launch_bounds__(TileShape<kSh>::threads, TileShape<kSh>::ctas)
   }
 }
 
-// cursor2[p] = off[p]; for a two-pass partition also the pass-1 bucket
-// starts cursor1[b] = bucket_off[b] = off[b << bits2] (bucket_off[B1] = n).
-__global__ void k_cursors(const uint64_t *__restrict__ off, uint32_t P, int bits2,
-                          uint32_t *__restrict__ cursor1, uint32_t *__restrict__ cursor2,
-                          uint64_t *__restrict__ bucket_off) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < P) {
-    cursor2[p] = (uint32_t)off[p];
-    if (cursor1 && (p & ((1u << bits2) - 1)) == 0) {
-      cursor1[p >> bits2] = (uint32_t)off[p];
-      bucket_off[p >> bits2] = off[p];
-    }
-  }
-  if (cursor1 && p == 0) bucket_off[P >> bits2] = off[P];
-}
-
-// Tiles of `tile` tuples per pass-1 bucket (the second pass's tile shape).
-__global__ void k_bucket_tiles(const uint64_t *__restrict__ bucket_off, uint32_t nb, uint32_t tile,
-                               uint64_t *__restrict__ tiles) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < nb) tiles[b] = (bucket_off[b + 1] - bucket_off[b] + tile - 1) / tile;
-}
-
 // ---------------------------------------------------------------- join
 
 // Work items per partition: ceil(|R_p| / rmax) build chunks times
-// ceil(|S_p| / w) probe chunks (zero when either side is empty).
-__global__ void k_join_items(const uint64_t *__restrict__ ro, const uint64_t *__restrict__ so,
-                             uint32_t P, uint32_t rmax, uint64_t w, uint64_t *__restrict__ items) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  const uint64_t nr = ro[p + 1] - ro[p], ns = so[p + 1] - so[p];
-  items[p] = (nr && ns) ? ((nr + rmax - 1) / rmax) * ((ns + w - 1) / w) : 0;
+// ceil(|S_p| / w) probe chunks (zero when either side is empty), as offsets;
+// the item counter and the results' start values beside them.
+__global__ void __launch_bounds__(1024)
+    k_join_plan(const uint64_t *__restrict__ ro, const uint64_t *__restrict__ so, uint32_t P, uint32_t rmax,
+                uint64_t w, uint64_t *__restrict__ items, unsigned long long *ctr, gbj::AggSpec spec, int64_t *out) {
+  __shared__ uint64_t s_scan[32];
+  if (threadIdx.x == 0) *ctr = 0;
+  if (threadIdx.x < (uint32_t)spec.n) out[threadIdx.x] = gbjd::agg_identity(spec.op[threadIdx.x]);
+  gbjd::cta_offsets(P, [&](uint32_t p) -> uint64_t {
+    const uint64_t nr = ro[p + 1] - ro[p], ns = so[p + 1] - so[p];
+    return nr && ns ? ((nr + rmax - 1) / rmax) * ((ns + w - 1) / w) : 0;
+  }, items, s_scan);
 }
 
 // Partition of work item `item`: largest p with item_off[p] <= item, where
@@ -912,12 +932,25 @@ int partition_impl(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint6
   constexpr int kPass = kHashOut ? kDigitPre : kDigit;
   const uint32_t P = 1u << bits, pmask = P - 1;
   Scratch scratch(ctx, s);
-  uint32_t *hist, *cursor2;
-  uint64_t *off;
+  const bool one = passes == 1 || (passes == 0 && bits <= 8);
+  const int bits2 = bits / 2, bits1 = bits - bits2;
+  const uint32_t B1 = 1u << bits1, m2 = (1u << bits2) - 1;
+  uint32_t *hist, *cursors;
+  uint64_t *off = offsets;
   GBJ_TRY(scratch.get(P + 1, &hist));
-  GBJ_TRY(scratch.get(P + 1, &cursor2));
-  GBJ_TRY(scratch.get(P + 1, &off));
-  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * P, s));
+  GBJ_TRY(scratch.get(P + B1, &cursors));
+  if (!off) GBJ_TRY(scratch.get(P + 1, &off));
+  PartPlan plan{off, cursors, nullptr, nullptr, nullptr, 0, 1};
+  int2 *tmp = nullptr;
+  if (!one) {
+    GBJ_TRY(scratch.get(B1 + 1, &plan.boff));
+    GBJ_TRY(scratch.get(B1 + 1, &plan.btiles));
+    plan.bcursor = cursors + P;
+    plan.bits2 = bits2;
+    plan.tile2 = tile_shape_for(m2 + 1, out_pairs != nullptr) == 0 ? TileShape<0>::tile : TileShape<1>::tile;
+    GBJ_TRY(scratch.get(n + 1, &tmp));
+  }
+  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * (P + 1), s));
   {
     const size_t smem = (size_t)P * sizeof(uint32_t);
     GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_pid_hist<kDigit>,
@@ -926,50 +959,23 @@ int partition_impl(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint6
     GBJ_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pid_hist<kDigit>, 1024, smem));
     const uint64_t grid = std::max<uint64_t>(
         1, std::min<uint64_t>((uint64_t)ctx->sm_count * std::max(per_sm, 1), (n + 16383) / 16384));
-    k_pid_hist<kDigit><<<(unsigned)grid, 1024, smem, s>>>(keys, n, shift, pmask, hist);
+    k_pid_hist<kDigit><<<(unsigned)grid, 1024, smem, s>>>(keys, n, shift, pmask, hist, plan);
     GBJ_TRY(after_launch(ctx, "k_pid_hist", s));
   }
-  GBJ_TRY(scan_u32_to_u64(ctx, hist, off, P, s));
-  if (passes == 1 || (passes == 0 && bits <= 8)) {
-    k_cursors<<<(P + 255) / 256, 256, 0, s>>>(off, P, 0, nullptr, cursor2, nullptr);
-    GBJ_TRY(after_launch(ctx, "k_cursors", s));
+  if (one) {
     if (out_pairs)
-      GBJ_TRY((launch_tile_pass<kPass, false, true, kHashOut>(ctx, keys, vals, nullptr, n, shift, pmask, nullptr,
-                                                              nullptr, 1, cursor2, out_pairs, nullptr, nullptr, s)));
-    else
-      GBJ_TRY((launch_tile_pass<kPass, false, false, false>(ctx, keys, vals, nullptr, n, shift, pmask, nullptr,
-                                                            nullptr, 1, cursor2, nullptr, out_keys, out_vals, s)));
-  } else {
-    const int bits2 = bits / 2, bits1 = bits - bits2;
-    const uint32_t B1 = 1u << bits1;
-    uint32_t *cursor1;
-    uint64_t *bucket_off, *tiles;
-    int2 *tmp;
-    GBJ_TRY(scratch.get(B1 + 1, &cursor1));
-    GBJ_TRY(scratch.get(B1 + 1, &bucket_off));
-    GBJ_TRY(scratch.get(B1 + 1, &tiles));
-    GBJ_TRY(scratch.get(n + 1, &tmp));
-    k_cursors<<<(P + 255) / 256, 256, 0, s>>>(off, P, bits2, cursor1, cursor2, bucket_off);
-    GBJ_TRY(after_launch(ctx, "k_cursors", s));
-    GBJ_TRY((launch_tile_pass<kPass, false, true, kHashOut>(ctx, keys, vals, nullptr, n, shift + bits2, B1 - 1,
-                                                            nullptr, nullptr, 1, cursor1, tmp, nullptr, nullptr,
-                                                            s)));
-    const uint32_t m2 = (1u << bits2) - 1;
-    const uint32_t tile2 = tile_shape_for(m2 + 1, out_pairs != nullptr) == 0 ? TileShape<0>::tile
-                                                                            : TileShape<1>::tile;
-    k_bucket_tiles<<<(B1 + 255) / 256, 256, 0, s>>>(bucket_off, B1, tile2, tiles);
-    GBJ_TRY(after_launch(ctx, "k_bucket_tiles", s));
-    GBJ_TRY(scan_u64(ctx, tiles, tiles, B1, s));
-    if (out_pairs)
-      GBJ_TRY((launch_tile_pass<kPass, true, true, false>(ctx, nullptr, nullptr, tmp, n, shift, m2, bucket_off,
-                                                          tiles, B1, cursor2, out_pairs, nullptr, nullptr, s)));
-    else
-      GBJ_TRY((launch_tile_pass<kPass, true, false, false>(ctx, nullptr, nullptr, tmp, n, shift, m2, bucket_off,
-                                                           tiles, B1, cursor2, nullptr, out_keys, out_vals, s)));
+      return launch_tile_pass<kPass, false, true, kHashOut>(ctx, keys, vals, nullptr, n, shift, pmask, nullptr,
+                                                            nullptr, 1, plan.cursor, out_pairs, nullptr, nullptr, s);
+    return launch_tile_pass<kPass, false, false, false>(ctx, keys, vals, nullptr, n, shift, pmask, nullptr, nullptr,
+                                                        1, plan.cursor, nullptr, out_keys, out_vals, s);
   }
-  if (offsets) GBJ_CHECK_CUDA(ctx, cudaMemcpyAsync(offsets, off, sizeof(uint64_t) * (P + 1),
-                                                   cudaMemcpyDeviceToDevice, s));
-  return GBJ_OK;
+  GBJ_TRY((launch_tile_pass<kPass, false, true, kHashOut>(ctx, keys, vals, nullptr, n, shift + bits2, B1 - 1, nullptr,
+                                                          nullptr, 1, plan.bcursor, tmp, nullptr, nullptr, s)));
+  if (out_pairs)
+    return launch_tile_pass<kPass, true, true, false>(ctx, nullptr, nullptr, tmp, n, shift, m2, plan.boff, plan.btiles,
+                                                      B1, plan.cursor, out_pairs, nullptr, nullptr, s);
+  return launch_tile_pass<kPass, true, false, false>(ctx, nullptr, nullptr, tmp, n, shift, m2, plan.boff, plan.btiles,
+                                                     B1, plan.cursor, nullptr, out_keys, out_vals, s);
 }
 
 }  // namespace
@@ -1069,8 +1075,7 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
   const bool by_rows = minor || (b_row && b_pay) || (p_row && p_pay);
   cudaStream_t s = pick_stream(ctx, stream);
   prof_mark(ctx, s);
-  GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
-  if (n_build == 0 || n_probe == 0) return GBJ_OK;
+  if (n_build == 0 || n_probe == 0) return init_agg_out(ctx, spec, d_out, s);
 
   // ---- plan: fewest radix bits whose largest expected build partition
   //      (mean + 5 sd) fits the on-chip table; explicit params override ----
@@ -1124,10 +1129,8 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
                            GBJ_DIGIT_HASH, 0, bits, R, nullptr, nullptr, ro, s, passes, true));
   GBJ_TRY(partition_tuples(ctx, d_probe_keys, p_pay && !by_rows ? d_probe_payload : nullptr, n_probe,
                            GBJ_DIGIT_HASH, 0, bits, S, nullptr, nullptr, so, s, passes, true));
-  k_join_items<<<(P + 255) / 256, 256, 0, s>>>(ro, so, P, kRMax, w, items);
-  GBJ_TRY(after_launch(ctx, "k_join_items", s));
-  GBJ_TRY(scan_u64(ctx, items, items, P, s));
-  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+  k_join_plan<<<1, 1024, 0, s>>>(ro, so, P, kRMax, w, items, ctr, spec, d_out);
+  GBJ_TRY(after_launch(ctx, "k_join_plan", s));
   const RowCols rc{minor ? d_build_minor : nullptr, minor ? d_probe_minor : nullptr,
                    b_pay ? d_build_payload : nullptr, p_pay ? d_probe_payload : nullptr};
   if (shape.threads == kJoinWide.threads)

@@ -10,16 +10,15 @@ constexpr int kThreads = 1024;
 constexpr int kPer = 4;
 constexpr uint64_t kTile = kThreads * kPer;
 
-template <typename In>
 __global__ void __launch_bounds__(kThreads)
-    k_scan_tiles(const In *in, uint64_t *out, uint64_t n, uint64_t *tile_sums) {
+    k_scan_tiles(const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *tile_sums) {
   __shared__ uint64_t warp_tot[32];
   const uint64_t base = blockIdx.x * kTile + (uint64_t)threadIdx.x * kPer;
   uint64_t v[kPer];
   uint64_t local = 0;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
-    v[j] = (base + j < n) ? (uint64_t)in[base + j] : 0;
+    v[j] = (base + j < n) ? in[base + j] : 0;
     local += v[j];
   }
   // inclusive warp scan of thread totals
@@ -66,8 +65,7 @@ __global__ void k_set_total(uint64_t *out, uint64_t n, const uint64_t *tile_off,
   out[n] = tile_off[ntiles];
 }
 
-template <typename In>
-int scan_impl(gbj_ctx *ctx, const In *in, uint64_t *out, uint64_t n,
+int scan_impl(gbj_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n,
               cudaStream_t s) {
   if (n == 0) {
     GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(out, 0, sizeof(uint64_t), s));
@@ -77,7 +75,7 @@ int scan_impl(gbj_ctx *ctx, const In *in, uint64_t *out, uint64_t n,
   Scratch scratch(ctx, s);
   uint64_t *sums;
   GBJ_TRY(scratch.get(ntiles + 1, &sums));
-  k_scan_tiles<In><<<(unsigned)ntiles, kThreads, 0, s>>>(in, out, n, sums);
+  k_scan_tiles<<<(unsigned)ntiles, kThreads, 0, s>>>(in, out, n, sums);
   GBJ_TRY(after_launch(ctx, "k_scan_tiles", s));
   if (ntiles == 1) {
     // single tile: its total is the grand total
@@ -85,7 +83,7 @@ int scan_impl(gbj_ctx *ctx, const In *in, uint64_t *out, uint64_t n,
     return after_launch(ctx, "k_set_total", s);
   }
   // sums[0..ntiles) -> exclusive offsets in place, sums[ntiles] = total
-  GBJ_TRY(scan_impl<uint64_t>(ctx, sums, sums, ntiles, s));
+  GBJ_TRY(scan_impl(ctx, sums, sums, ntiles, s));
   k_scan_add<<<(unsigned)ntiles, kThreads, 0, s>>>(out, n, sums);
   GBJ_TRY(after_launch(ctx, "k_scan_add", s));
   k_set_total<<<1, 1, 0, s>>>(out, n, sums, ntiles);
@@ -96,12 +94,7 @@ int scan_impl(gbj_ctx *ctx, const In *in, uint64_t *out, uint64_t n,
 
 int scan_u64(gbj_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n,
              cudaStream_t s) {
-  return scan_impl<uint64_t>(ctx, in, out, n, s);
-}
-
-int scan_u32_to_u64(gbj_ctx *ctx, const uint32_t *in, uint64_t *out,
-                    uint64_t n, cudaStream_t s) {
-  return scan_impl<uint32_t>(ctx, in, out, n, s);
+  return scan_impl(ctx, in, out, n, s);
 }
 
 }  // namespace gbj
