@@ -259,7 +259,7 @@ int gbj_radix_join_count_i64(gbj_ctx *ctx, const int64_t *d_r_keys, uint64_t nr,
  * is 0 or the join kernel's 1024 threads. */
 typedef struct gbj_radix_params {
   int32_t bits;       /* radix bits, 0 = autotuned                        */
-  int32_t passes;     /* 1 or 2, 0 = one pass up to 8 bits, two above     */
+  int32_t passes;     /* 1 or 2, 0 = one pass up to 12 bits, two above    */
   int32_t block;      /* threads per block of the join kernel, 0 = auto   */
   int32_t log_parts;  /* plan field log_parts (reference: 13), 0 = unset  */
 } gbj_radix_params;

@@ -21,10 +21,11 @@
 //    writes 128 regions; the second writes inside one 32 MB bucket).  The
 //    pass is software-pipelined: a CTA issues the next tile's loads as soon
 //    as the current tile sits in shared memory, and the output-range atomic
-//    is in flight while the tile is scattered on chip;
+//    is in flight while the tile is scattered on chip.  Fan-outs of 2^9 to
+//    2^12 take one pass with larger tiles (k_wide_pass);
 //  * radix bits are chosen so the largest build partition fits an on-chip
-//    table of kRMax tuples (the bench's 2^27-row side: 16384 partitions of
-//    8192 +- 90 tuples);
+//    table of kRMax tuples (a 2^27-row side: 16384 partitions of 8192 +- 90
+//    tuples) and every SM gets work;
 //  * the join kernel is persistent: CTAs pull work items (partition, build
 //    chunk, probe chunk) from an atomic counter, so a skewed probe partition
 //    (Zipf keys) is spread over many SMs.  The on-chip table stores keys and
@@ -411,6 +412,147 @@ __global__ void __launch_bounds__(TileShape<kSh>::threads, TileShape<kSh>::ctas)
         } else {
           out_k[g] = v.x;
           out_v[g] = v.y;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// A pass of 9 to 12 digit bits over the input columns, instead of two passes
+// over half of the bits each: one CTA of 1024 threads per SM sorts tiles of
+// kPer * 1024 tuples, so that a tile still has three or more tuples of a digit
+// and its runs are written in whole sectors.  One shared histogram for the CTA
+// (a row per warp would not fit) gives every tuple its rank; more than 4096
+// digits would leave runs of one or two tuples.
+//
+// What bounds it is the shared-memory pipe and the phases of the one CTA that
+// follow one another.  Measured on GB300, 2^27 keys with row positions (ms;
+// two passes: 0.88): 9 bits 0.44, 10 bits 0.48, 11 bits 0.51, 12 bits 0.61, 13
+// bits 0.93, 14 bits 1.46; with a value column 8 tuples a thread are faster
+// than 12, which spill (9 to 12 bits 0.47, 0.54, 0.64, 0.78; two passes 0.93).
+constexpr int kWideBits = 12;
+constexpr int kWideThreads = 1024;
+
+template <int kPer>
+struct WideSmem {
+  int2 sorted[kWideThreads * kPer];
+  uint32_t start[1 << kWideBits];   // counts, then where a digit starts in the tile
+  uint32_t gdelta[1 << kWideBits];  // output position of sorted[i] = gdelta[digit] + i
+  uint32_t wsum[kWideThreads / 32];
+};
+
+template <int kDigit, bool kAoSOut, bool kHashLoad, bool kVals>
+__global__ void __launch_bounds__(kWideThreads, 1)
+    k_wide_pass(const int32_t *__restrict__ keys, const int32_t *__restrict__ vals, uint32_t n, int dshift,
+                uint32_t dmask, uint32_t *__restrict__ cursor, int2 *__restrict__ out_pairs,
+                int32_t *__restrict__ out_k, int32_t *__restrict__ out_v) {
+  constexpr int kPer = kVals ? 8 : 12;
+  constexpr uint32_t kTile = kWideThreads * kPer;
+  constexpr int kDigits = (1 << kWideBits) / kWideThreads;  // of a thread, at most
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  WideSmem<kPer> &S = *reinterpret_cast<WideSmem<kPer> *>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t ndig = dmask + 1, ntiles = (n + kTile - 1) / kTile;
+  int32_t next[kPer];
+  auto load_tile = [&](uint32_t t) {
+    const uint32_t lo = t * kTile;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t i = lo + tid + j * kWideThreads;
+      next[j] = i < n ? __ldcs(keys + i) : 0;
+    }
+  };
+  uint32_t t = blockIdx.x;
+  if (t < ntiles) load_tile(t);
+  for (uint32_t d = tid; d < ndig; d += kWideThreads) S.start[d] = 0;
+  __syncthreads();
+  for (; t < ntiles; t += gridDim.x) {
+    const uint32_t lo = t * kTile, cnt = n - lo < kTile ? n - lo : kTile;
+    int32_t key[kPer], val[kVals ? kPer : 1];
+    uint32_t rank[kPer / 2];  // 16 bits each
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      key[j] = kHashLoad ? (int32_t)gbjd::fmix32((uint32_t)next[j]) : next[j];
+      uint32_t r = 0;
+      if (tid + j * kWideThreads < cnt) r = atomicAdd(&S.start[digit_of<kDigit>(key[j], dshift, dmask)], 1u);
+      if (j & 1) rank[j / 2] |= r << 16;
+      else rank[j / 2] = r;
+    }
+    if (kVals) {  // in flight through the scan
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        const uint32_t i = tid + j * kWideThreads;
+        val[kVals ? j : 0] = i < cnt ? __ldcs(vals + lo + i) : 0;
+      }
+    }
+    __syncthreads();
+    // a thread's digits for the scan are neighbours
+    uint32_t c[kDigits], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kDigits; ++j) {
+      const uint32_t d = tid * kDigits + j;
+      c[j] = d < ndig ? S.start[d] : 0;
+      sum += c[j];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) S.wsum[warp] = incl;
+    __syncthreads();
+    uint32_t before = lane < warp ? S.wsum[lane] : 0;
+    before = __reduce_add_sync(0xffffffffu, before);
+    uint32_t run = before + incl - sum;
+#pragma unroll
+    for (int j = 0; j < kDigits; ++j) {
+      const uint32_t d = tid * kDigits + j;
+      if (d < ndig) S.start[d] = run;
+      run += c[j];
+    }
+    __syncthreads();
+    // and for the cursors neighbouring threads have neighbouring digits
+    uint32_t gpos[kDigits], st[kDigits];
+#pragma unroll
+    for (int j = 0; j < kDigits; ++j) {
+      const uint32_t d = j * kWideThreads + tid;
+      gpos[j] = st[j] = 0;
+      if (d < ndig) {
+        st[j] = S.start[d];
+        const uint32_t end = d + 1 < ndig ? S.start[d + 1] : cnt;
+        if (end > st[j]) gpos[j] = atomicAdd(&cursor[d], end - st[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t i = tid + j * kWideThreads;
+      if (i < cnt) {
+        const uint32_t r = j & 1 ? rank[j / 2] >> 16 : rank[j / 2] & 0xffffu;
+        S.sorted[S.start[digit_of<kDigit>(key[j], dshift, dmask)] + r] =
+            make_int2(key[j], kVals ? val[kVals ? j : 0] : (int32_t)(lo + i));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kDigits; ++j) {
+      const uint32_t d = j * kWideThreads + tid;
+      if (d < ndig) S.gdelta[d] = gpos[j] - st[j];
+    }
+    if (t + gridDim.x < ntiles) load_tile(t + gridDim.x);
+    __syncthreads();
+    for (uint32_t d = tid; d < ndig; d += kWideThreads) S.start[d] = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t i = tid + j * kWideThreads;
+      if (i < cnt) {
+        const int2 x = S.sorted[i];
+        const uint32_t g = S.gdelta[digit_of<kDigit>(x.x, dshift, dmask)] + i;
+        if (kAoSOut) {
+          out_pairs[g] = x;
+        } else {
+          out_k[g] = x.x;
+          out_v[g] = x.y;
         }
       }
     }
@@ -916,6 +1058,29 @@ int launch_tile_pass(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, con
                                                                      s);
 }
 
+template <int kDigit, bool kAoSOut, bool kHashLoad, bool kVals>
+int launch_wide_pass_v(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint64_t n, int dshift, uint32_t dmask,
+                       uint32_t *cursor, int2 *op, int32_t *ok, int32_t *ov, cudaStream_t s) {
+  constexpr int kPer = kVals ? 8 : 12;
+  auto kern = k_wide_pass<kDigit, kAoSOut, kHashLoad, kVals>;
+  constexpr size_t smem = sizeof(WideSmem<kPer>);
+  GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const uint64_t tiles = (n + kWideThreads * kPer - 1) / (kWideThreads * kPer);
+  kern<<<(unsigned)std::min<uint64_t>(tiles, ctx->sm_count), kWideThreads, smem, s>>>(keys, vals, (uint32_t)n, dshift,
+                                                                                      dmask, cursor, op, ok, ov);
+  return after_launch(ctx, "k_wide_pass", s);
+}
+
+template <int kDigit, bool kAoSOut, bool kHashLoad>
+int launch_wide_pass(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint64_t n, int dshift, uint32_t dmask,
+                     uint32_t *cursor, int2 *op, int32_t *ok, int32_t *ov, cudaStream_t s) {
+  if (vals)
+    return launch_wide_pass_v<kDigit, kAoSOut, kHashLoad, true>(ctx, keys, vals, n, dshift, dmask, cursor, op, ok, ov,
+                                                                s);
+  return launch_wide_pass_v<kDigit, kAoSOut, kHashLoad, false>(ctx, keys, vals, n, dshift, dmask, cursor, op, ok, ov,
+                                                               s);
+}
+
 // kHashOut: the tuples leave with fmix32(key) in place of the key (the
 // partitioned join's layout; AoS output only), and the passes take their
 // digits from that word.
@@ -932,7 +1097,8 @@ int partition_impl(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint6
   constexpr int kPass = kHashOut ? kDigitPre : kDigit;
   const uint32_t P = 1u << bits, pmask = P - 1;
   Scratch scratch(ctx, s);
-  const bool one = passes == 1 || (passes == 0 && bits <= 8);
+  const bool wide = passes == 0 && bits > 8 && bits <= kWideBits;
+  const bool one = wide || passes == 1 || (passes == 0 && bits <= 8);
   const int bits2 = bits / 2, bits1 = bits - bits2;
   const uint32_t B1 = 1u << bits1, m2 = (1u << bits2) - 1;
   uint32_t *hist, *cursors;
@@ -961,6 +1127,13 @@ int partition_impl(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint6
         1, std::min<uint64_t>((uint64_t)ctx->sm_count * std::max(per_sm, 1), (n + 16383) / 16384));
     k_pid_hist<kDigit><<<(unsigned)grid, 1024, smem, s>>>(keys, n, shift, pmask, hist, plan);
     GBJ_TRY(after_launch(ctx, "k_pid_hist", s));
+  }
+  if (wide) {
+    if (out_pairs)
+      return launch_wide_pass<kPass, true, kHashOut>(ctx, keys, vals, n, shift, pmask, plan.cursor, out_pairs, nullptr,
+                                                     nullptr, s);
+    return launch_wide_pass<kPass, false, false>(ctx, keys, vals, n, shift, pmask, plan.cursor, nullptr, out_keys,
+                                                 out_vals, s);
   }
   if (one) {
     if (out_pairs)
@@ -1077,25 +1250,48 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
   prof_mark(ctx, s);
   if (n_build == 0 || n_probe == 0) return init_agg_out(ctx, spec, d_out, s);
 
-  // ---- plan: fewest radix bits whose largest expected build partition
-  //      (mean + 5 sd) fits the on-chip table; explicit params override ----
+  // ---- plan: the fewest radix bits whose largest expected build partition
+  //      (mean + 5 sd) fits the on-chip table, but enough partitions to give
+  //      every CTA a few work items; explicit params override ----
   const int passes = params ? params->passes : 0;
-  // join kernel shape: the caller's block size, else an autotuned one, else
-  // two 512-thread blocks per SM
+  auto fit_bits = [&](int rmax) {
+    int b = 1;
+    while (b < kMaxPartBits) {
+      const double mean = (double)n_build / (double)(1u << b);
+      if (mean + 5.0 * std::sqrt(mean) <= (double)rmax) break;
+      ++b;
+    }
+    return b;
+  };
+  // 256 to 1024 partitions of about 2^14 tuples of both sides: fewer leave
+  // SMs without work (2^16 and 2^20 rows: 4 bits 219 us, 8 bits 69), more
+  // cost a table set-up of 4 us each (12 bits at 2^20 and 2^24 rows 260 us, 10
+  // bits 200, 8 bits 316)
+  const int even = std::max(8, std::min(10, log2_ceil((n_build + n_probe) >> 14)));
+  // Join kernel shape: the caller's block size, else an autotuned one, else
+  // two 512-thread blocks per SM while its partitions are small enough at 10
+  // bits, else 1024 threads, which take twice the tuples and so one radix bit
+  // less (us; 4 M and 128 M rows: 512 threads at 10 bits 1144, at 11 bits
+  // 1076, 1024 threads at 10 bits 1080; 16 M and 64 M: 512 at 12 bits 799,
+  // 1024 at 11 bits 752; 30 M and 128 M: 512 at 13 bits, two passes, 1758,
+  // 1024 at 12 bits 1478; 2^27 and 2^29: 15 bits 7631, 14 bits 7162).
+  constexpr int kPairRoom = 3900;  // a fuller 512-thread table loses more than a bit costs
+  const bool explicit_bits = params && (params->log_parts > 0 || params->bits > 0);
   int block = params ? params->block : 0;
   if (!block) {
     const int32_t tb = tuned_value(ctx, tune_key("radixblock", n_build, n_probe));
-    block = tb > 0 ? tb : kJoinPair.threads;
+    if (tb > 0) {
+      block = tb;
+    } else if (explicit_bits) {
+      const int b = params->bits > 0 ? params->bits : params->log_parts;
+      block = fit_bits(kJoinPair.rmax) <= b ? kJoinPair.threads : kJoinWide.threads;
+    } else {
+      block = std::max(fit_bits(kPairRoom), even) <= 10 ? kJoinPair.threads : kJoinWide.threads;
+    }
   }
   const JoinShape shape = block == kJoinWide.threads ? kJoinWide : kJoinPair;
   const uint32_t kRMax = (uint32_t)shape.rmax;
-  int bits = 1;
-  while (bits < kMaxPartBits) {
-    const double mean = (double)n_build / (double)(1u << bits);
-    if (mean + 5.0 * std::sqrt(mean) <= (double)kRMax) break;
-    ++bits;
-  }
-  const bool explicit_bits = params && (params->log_parts > 0 || params->bits > 0);
+  int bits = std::max(even, fit_bits(shape.threads == kJoinPair.threads ? kPairRoom : shape.rmax));
   if (!explicit_bits) {  // an autotuned choice for this size bucket, if any
     const int32_t tb = tuned_value(ctx, tune_key(shape.threads == kJoinWide.threads ? "radix" : "radix512",
                                                  n_build, n_probe));

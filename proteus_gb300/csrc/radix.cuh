@@ -10,8 +10,8 @@ constexpr int kMaxPartBits = 15;
 // into a contiguous, partition-major output.  vals == nullptr carries the
 // row position.  Output either AoS (out_pairs != nullptr, int2 {key, val})
 // or SoA (out_keys / out_vals).  offsets gets 2^bits + 1 entries.
-// One histogram pass, then one tile pass per digit group; tuples keep no
-// particular order inside a partition.  passes: 0 = one pass up to 8 bits,
+// One histogram pass, then one pass per digit group; tuples keep no
+// particular order inside a partition.  passes: 0 = one pass up to 12 bits,
 // two above; 1 = one pass (bits <= 8); 2 = two passes (bits >= 2).
 // hash_out (GBJ_DIGIT_HASH, AoS output only): each tuple leaves with
 // fmix32(key) in place of the key, as the partitioned join consumes them.
