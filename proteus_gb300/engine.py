@@ -26,10 +26,11 @@ def _cur_stream():
     """torch's current stream as a cudaStream_t for the ABI.  torch reports
     its default stream as handle 0, which the ABI reads as "the context's own
     stream"; pass cudaStreamLegacy instead so library kernels stay ordered
-    with torch's copies on that stream."""
+    with torch's copies on that stream.  (Asked for as a raw handle: building
+    a torch.cuda.Stream object costs 3 us, as much as a kernel launch.)"""
     import torch
 
-    return torch.cuda.current_stream().cuda_stream or CUDA_STREAM_LEGACY
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) or CUDA_STREAM_LEGACY
 
 
 class Table:
