@@ -207,6 +207,7 @@ int validate_aggs(gbj_ctx *ctx, const gbj_agg *aggs, int32_t n_aggs) {
 }
 
 __global__ void k_init_agg_out(AggSpec s, int64_t *out) {
+  asm volatile("griddepcontrol.launch_dependents;");  // launch_behind_init
   int j = threadIdx.x;
   if (j < s.n) out[j] = gbjd::agg_identity(s.op[j]);
 }

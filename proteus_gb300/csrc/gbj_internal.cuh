@@ -158,6 +158,25 @@ AggSpec make_spec(const gbj_agg *aggs, int32_t n_aggs);
 int init_agg_out(gbj_ctx *ctx, const AggSpec &spec, int64_t *d_out,
                  cudaStream_t s);
 
+// Launches a kernel right behind init_agg_out on the same stream without
+// waiting for it: the kernel starts while the identities are written (a
+// launch and 2 us of a kernel that is otherwise latency), and
+// gbjd::after_init() before its first access to them waits for that launch.
+// Everything before init_agg_out has ended when either starts.
+template <typename... Params, typename... Args>
+void launch_behind_init(void (*kernel)(Params...), unsigned grid, unsigned block, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // errors: after_launch
+}
+
 }  // namespace gbj
 
 // ---------------------------------------------------------- device helpers
@@ -186,6 +205,10 @@ __host__ __device__ __forceinline__ uint32_t fmix32_inv(uint32_t h) {
   h ^= h >> 16;
   return h;
 }
+
+// Waits for the kernel this one was launched behind (launch_behind_init);
+// nothing to wait for after an ordinary launch.
+__device__ __forceinline__ void after_init() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void latch(uint32_t *status, uint32_t bit) {
   atomicOr(status, bit);

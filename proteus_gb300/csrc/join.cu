@@ -165,10 +165,10 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ------------------------------------------------ bucketed join table
-// The table gbj_join_build makes: buckets of four slots, 32 bytes each --
-// four keys then four values (the build payload, or row + 1 when the build
-// side has none) -- so a probe reads one L2 sector per bucket and finds the
-// key and its payload without a second, dependent load.  Keys are stored
+// The table gbj_join_build makes: buckets of four slots, 32 bytes each -- a
+// slot is {key, value} (the build payload, or row + 1 when the build side has
+// none) and is claimed by one 64-bit CAS -- so a probe reads one L2 sector per
+// bucket and finds the key and its payload without a second, dependent load.  Keys are stored
 // xor INT32_MIN, so the all-zero word of a cleared table marks an empty
 // slot; build rows whose key is INT32_MIN (stored word 0) go to a side list
 // instead.  A table with a payload keeps row + 1 of every slot in a
@@ -188,9 +188,9 @@ __global__ void __launch_bounds__(kThreads)
 #define GBJ_JB_GROUP 4
 #endif
 constexpr int kJbGroup = GBJ_JB_GROUP;
+// In memory: {key ^ INT32_MIN (0 = empty), payload or row + 1} four times.
 struct __align__(32) JBucket {
-  int4 k;  // key ^ INT32_MIN, 0 = empty
-  int4 x;  // payload, or row + 1
+  int4 k, x;  // as loaded
 };
 
 // One bucket in a single 256-bit load (ld.global.nc.v8, sm_100 and later):
@@ -198,7 +198,7 @@ struct __align__(32) JBucket {
 __device__ __forceinline__ JBucket ld_bucket(const JBucket *p) {
   JBucket r;
   asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-      : "=r"(r.k.x), "=r"(r.k.y), "=r"(r.k.z), "=r"(r.k.w), "=r"(r.x.x), "=r"(r.x.y), "=r"(r.x.z), "=r"(r.x.w)
+      : "=r"(r.k.x), "=r"(r.x.x), "=r"(r.k.y), "=r"(r.x.y), "=r"(r.k.z), "=r"(r.x.z), "=r"(r.k.w), "=r"(r.x.w)
       : "l"(p));
   return r;
 }
@@ -213,47 +213,94 @@ __device__ __forceinline__ uint32_t hits4(const int4 &k, int32_t kf) {
 }
 __device__ __forceinline__ bool room4(const int4 &k) { return (k.x == 0) | (k.y == 0) | (k.z == 0) | (k.w == 0); }
 
-// meta[0]: a duplicate build key was seen; meta[1]: side-list length.  A
-// row claims the first free slot of its home bucket, starting at a slot
-// chosen by the top hash bits, then of the following buckets.
+// A row's slot in a table at `bk` (global or shared memory): it claims the
+// first free slot of its home bucket, starting at a slot chosen by the top
+// hash bits, then of the following buckets.  rows may be null.  False: full.
+__device__ __forceinline__ unsigned long long jb_word(int32_t kf, int32_t value) {
+  return ((unsigned long long)(uint32_t)value << 32) | (uint32_t)kf;
+}
+__device__ __forceinline__ bool jb_place(unsigned long long *bk, int32_t *rows, uint32_t bmask, uint32_t h, int32_t kf,
+                                         int32_t value, int32_t row1, bool &dup) {
+  uint32_t b = h & bmask;
+  const uint32_t o = h >> 30;  // start slot (high bits, independent of the bucket for 2^30 buckets or fewer)
+  for (uint32_t step = 0; step <= bmask; ++step) {
+#pragma unroll 1
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint64_t sl = 4ull * b + ((o + j) & 3u);
+      const unsigned long long old = atomicCAS(&bk[sl], 0ull, jb_word(kf, value));
+      if (old == 0) {
+        if (rows) rows[sl] = row1;
+        return true;
+      }
+      dup |= (int32_t)(uint32_t)old == kf;
+    }
+    b = (b + 1) & bmask;
+  }
+  return false;
+}
+
+// meta[0]: a duplicate build key was seen; meta[1]: side-list length.  One
+// row at a time per thread: two or four claims in flight together were slower
+// (2^20 rows 48, 50, 77 us; 2^22 rows 178, 205, 323).
 __global__ void __launch_bounds__(kThreads)
     k_jb_build(const int32_t *__restrict__ keys, const int32_t *__restrict__ payload, uint64_t n,
-               JBucket *__restrict__ bk, int4 *__restrict__ rows, uint32_t bmask, uint32_t *__restrict__ meta,
-               int32_t *__restrict__ side, uint32_t *status) {
+               unsigned long long *__restrict__ bk, int32_t *__restrict__ rows, uint32_t bmask,
+               uint32_t *__restrict__ meta, int32_t *__restrict__ side, uint32_t *status) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   bool dup = false;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int32_t key = keys[i];
-    const int32_t pv = payload ? payload[i] : (int32_t)(i + 1);
-    const int32_t kf = key ^ kKeyFlip;
-    if (kf == 0) {  // INT32_MIN: the side list
-      side[atomicAdd(&meta[1], 1u)] = (int32_t)i;
-      continue;
-    }
-    const uint32_t h = gbjd::fmix32((uint32_t)key);
-    uint32_t b = h & bmask;
-    const uint32_t o = h >> 30;  // start slot (high bits, independent of the bucket for 2^30 buckets or fewer)
-    bool placed = false;
-    for (uint32_t step = 0; step <= bmask && !placed; ++step) {
-      int32_t *kw = reinterpret_cast<int32_t *>(&bk[b].k);
-#pragma unroll
-      for (uint32_t j = 0; j < 4; ++j) {
-        if (placed) break;
-        const uint32_t sl = (o + j) & 3u;
-        const int32_t old = atomicCAS(&kw[sl], 0, kf);
-        if (old == 0) {
-          reinterpret_cast<int32_t *>(&bk[b].x)[sl] = pv;
-          if (rows) reinterpret_cast<int32_t *>(&rows[b])[sl] = (int32_t)(i + 1);
-          placed = true;
-        } else {
-          dup |= old == kf;
-        }
-      }
-      b = (b + 1) & bmask;
-    }
-    if (!placed) gbjd::latch(status, GBJ_DEV_CAPACITY);
+    const int32_t key = keys[i], kf = key ^ kKeyFlip;
+    const int32_t val = payload ? payload[i] : (int32_t)(i + 1);
+    if (kf == 0) side[atomicAdd(&meta[1], 1u)] = (int32_t)i;  // INT32_MIN: the side list
+    else if (!jb_place(bk, rows, bmask, gbjd::fmix32((uint32_t)key), kf, val, (int32_t)(i + 1), dup))
+      gbjd::latch(status, GBJ_DEV_CAPACITY);
   }
   if (dup) meta[0] = 1;
+}
+
+// A small table (at most kSmallSlots slots) in one CTA: built in shared memory
+// and written out whole, so that it needs no clearing before it and no chain
+// of L2 atomics.  Build, start values and 60,000 probes on the GPU, 100, 1000
+// and 4000 rows with payloads: 16.6, 18.6, 25.0 us; cleared and built in L2
+// 20.7, 26.7, 30.8 us.
+constexpr int kSmallThreads = 1024;
+constexpr uint32_t kSmallSlots = 8192;
+
+__global__ void __launch_bounds__(kSmallThreads)
+    k_jb_build_small(const int32_t *__restrict__ keys, const int32_t *__restrict__ payload, uint32_t n,
+                     uint4 *__restrict__ bk, uint4 *__restrict__ rows, uint32_t slots, uint32_t *__restrict__ meta,
+                     int32_t *__restrict__ side) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned long long *s_bk = reinterpret_cast<unsigned long long *>(smem);
+  int32_t *s_rows = rows ? reinterpret_cast<int32_t *>(s_bk + slots) : nullptr;
+  __shared__ uint32_t s_meta[2];
+  constexpr int kPer = kSmallSlots / 2 / kSmallThreads;  // rows of a thread, at most
+  int32_t key[kPer], val[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const uint32_t i = threadIdx.x + u * kSmallThreads;
+    key[u] = i < n ? __ldg(keys + i) : 0;
+    val[u] = payload ? (i < n ? __ldg(payload + i) : 0) : (int32_t)(i + 1);
+  }
+  const uint32_t words = slots * (rows ? 12 : 8) / 16;
+  for (uint32_t i = threadIdx.x; i < words; i += kSmallThreads) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
+  if (threadIdx.x < 2) s_meta[threadIdx.x] = 0;
+  __syncthreads();
+  bool dup = false;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const uint32_t i = threadIdx.x + u * kSmallThreads;
+    if (i >= n) continue;
+    const int32_t kf = key[u] ^ kKeyFlip;
+    if (kf == 0) side[atomicAdd(&s_meta[1], 1u)] = (int32_t)i;
+    else jb_place(s_bk, s_rows, slots / 4 - 1, gbjd::fmix32((uint32_t)key[u]), kf, val[u], (int32_t)(i + 1), dup);  // 2 n slots
+  }
+  if (dup) s_meta[0] = 1;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < slots / 2; i += kSmallThreads) bk[i] = reinterpret_cast<const uint4 *>(s_bk)[i];
+  if (rows)
+    for (uint32_t i = threadIdx.x; i < slots / 4; i += kSmallThreads) rows[i] = reinterpret_cast<const uint4 *>(s_rows)[i];
+  if (threadIdx.x < 2) meta[threadIdx.x] = s_meta[threadIdx.x];
 }
 
 // Probe with fused aggregate over the bucketed table.  A probe visits its
@@ -320,7 +367,6 @@ __global__ void __launch_bounds__(kThreads, GBJ_JB_MIN_BLOCKS)
       a_cnt += 1;
       if (kAgg == kAggCountProduct) a_sum += (kPay ? (int64_t)bpay[r] : 0) * pv;
       else a_sum += (int64_t)r ^ (int64_t)prow;
-      if (unique) break;
     }
   };
   auto finish = [&](int32_t k, int64_t pv, uint64_t prow, uint32_t b, const JBucket &e) {
@@ -377,6 +423,7 @@ __global__ void __launch_bounds__(kThreads, GBJ_JB_MIN_BLOCKS)
   acc.init(spec);
   acc.v[0] = a_cnt;
   acc.v[1] = a_sum;
+  gbjd::after_init();
   gbjd::block_flush(spec, acc, red, out);
 }
 
@@ -410,7 +457,6 @@ __global__ void __launch_bounds__(kThreads)
     if (kf == 0) {
       for (uint32_t s = 0; s < nside; ++s) {
         emit(side[s], pr);
-        if (unique) break;
       }
       continue;
     }
@@ -442,8 +488,7 @@ __global__ void __launch_bounds__(kThreads)
 // (core/olap/lib/expressions/expressions-hasher.cpp:66-84).
 struct __align__(32) JBucket64 {
   unsigned long long k[2];
-  int32_t x[2];  // build payload (0 without one)
-  int32_t r[2];  // row + 1
+  int2 x[2];  // {build payload (0 without one), row + 1}
 };
 constexpr unsigned long long kFlip64 = 0x8000000000000000ull;
 
@@ -464,8 +509,8 @@ __device__ __forceinline__ JBucket64 ld_bucket64(const JBucket64 *p) {
   JBucket64 b;
   b.k[0] = ((unsigned long long)w[1] << 32) | w[0];
   b.k[1] = ((unsigned long long)w[3] << 32) | w[2];
-  b.x[0] = (int32_t)w[4], b.x[1] = (int32_t)w[5];
-  b.r[0] = (int32_t)w[6], b.r[1] = (int32_t)w[7];
+  b.x[0] = make_int2((int32_t)w[4], (int32_t)w[5]);
+  b.x[1] = make_int2((int32_t)w[6], (int32_t)w[7]);
   return b;
 }
 
@@ -495,8 +540,7 @@ __global__ void __launch_bounds__(kThreads)
         const uint32_t sl = (o + j) & 1u;
         const unsigned long long old = atomicCAS(&bk[b].k[sl], 0ull, kf);
         if (old == 0) {
-          bk[b].x[sl] = pv;
-          bk[b].r[sl] = (int32_t)(i + 1);
+          bk[b].x[sl] = make_int2(pv, (int32_t)(i + 1));
           placed = true;
         } else {
           dup |= old == kf;
@@ -551,9 +595,9 @@ struct JLayout64 {
     return (uint32_t)(e.k[0] == w) | ((uint32_t)(e.k[1] == w) << 1);
   }
   static __device__ __forceinline__ bool room(const Bucket &e) { return (e.k[0] == 0) | (e.k[1] == 0); }
-  static __device__ __forceinline__ int32_t value(const Bucket &e, uint32_t i) { return i ? e.x[1] : e.x[0]; }
+  static __device__ __forceinline__ int32_t value(const Bucket &e, uint32_t i) { return i ? e.x[1].x : e.x[0].x; }
   static __device__ __forceinline__ int32_t row(const JTable &, const Bucket &e, uint32_t, uint32_t i) {
-    return (i ? e.r[1] : e.r[0]) - 1;
+    return (i ? e.x[1].y : e.x[0].y) - 1;
   }
 };
 
@@ -687,7 +731,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
         srow = __ldg(t.side + b);
         ++b;
         hits = 1;
-        go_on = left != 0 && !unique;
+        go_on = left != 0;
       } else {
         b = (b + 1) & t.bmask;
         e = L::load(t, b);
@@ -734,6 +778,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
   gbjd::Acc acc;
 #pragma unroll
   for (int j = 0; j < GBJ_MAX_AGGS; ++j) acc.v[j] = j < kMaxA ? v[j < kMaxA ? j : 0] : 0;
+  gbjd::after_init();
   gbjd::block_flush(spec, acc, red, out);
 }
 
@@ -765,7 +810,6 @@ __global__ void __launch_bounds__(kThreads)
     if (kf == 0) {
       for (uint32_t s = 0; s < nside; ++s) {
         emit(side[s], pr);
-        if (unique) break;
       }
       continue;
     }
@@ -775,7 +819,7 @@ __global__ void __launch_bounds__(kThreads)
       bool stop = e.k[0] == 0 || e.k[1] == 0;
       for (int j = 0; j < 2; ++j) {
         if (e.k[j] == kf) {
-          emit(e.r[j] - 1, pr);
+          emit(e.x[j].y - 1, pr);
           if (unique) stop = true;
         }
       }
@@ -798,6 +842,7 @@ __global__ void __launch_bounds__(kThreads)
     const int64_t v = col ? col[r] : 0;
     acc.update(spec, (int32_t)v, v, v, r, r);
   }
+  gbjd::after_init();
   gbjd::block_flush(spec, acc, red, out);
 }
 
@@ -864,12 +909,9 @@ template <typename L>
 void launch_jb_list(int sm_count, const gbj_table *t, uint64_t nbk, const typename L::Key *keys, const int32_t *pay,
                     uint64_t n, const gbj::AggSpec &spec, int64_t *out, cudaStream_t s) {
   const JTable jt{t->slots, t->rows, (uint32_t)(nbk - 1), t->payload, t->meta, t->side};
-  if (spec.n <= 4)
-    k_jb_probe_list<L, 4><<<grid_for_sms(sm_count, n, kListThreads, kListCtas), kListThreads, 0, s>>>(keys, pay, n, jt, spec,
-                                                                                            out);
-  else
-    k_jb_probe_list<L, 8><<<grid_for_sms(sm_count, n, kListThreads, kListCtas), kListThreads, 0, s>>>(keys, pay, n, jt, spec,
-                                                                                            out);
+  const int grid = grid_for_sms(sm_count, n, kListThreads, kListCtas);
+  launch_behind_init(spec.n <= 4 ? k_jb_probe_list<L, 4> : k_jb_probe_list<L, 8>, grid, kListThreads, s, keys, pay, n,
+                     jt, spec, out);
 }
 
 // Probe kernel over a bucketed table: 16-byte probe loads when both probe
@@ -889,9 +931,9 @@ void launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, co
   }
   const int gv = grid_for_sms(sm_count, (n + kJbGroup - 1) / kJbGroup, kThreads, 2);
   const int gs = grid_for_sms(sm_count, n, kThreads);
-#define GBJ_JB_PROBE(V, A)                                                                               \
-  k_jb_probe_agg<V, A, kPay><<<V ? gv : gs, kThreads, 0, s>>>(keys, pay, n, bk, t->rows, bmask, t->payload, \
-                                                              t->meta, t->side, spec, out)
+#define GBJ_JB_PROBE(V, A)                                                                                  \
+  launch_behind_init(k_jb_probe_agg<V, A, kPay>, V ? gv : gs, kThreads, s, keys, pay, n, bk, t->rows, bmask, \
+                     t->payload, t->meta, t->side, spec, out)
   if (vec) {
     if (is_xor) GBJ_JB_PROBE(true, kAggCountXor);
     else GBJ_JB_PROBE(true, kAggCountProduct);
@@ -1018,22 +1060,30 @@ int gbj_join_build(gbj_ctx *ctx, const int32_t *d_keys,
   t->keys = d_keys;
   t->payload = d_payload;
   t->n = n;
-  cudaError_t e = cudaMemsetAsync(mem, 0, clear_bytes, s);
-  if (e != cudaSuccess) {
+  auto fail = [&](int code) {
     pool_release(ctx, mem, s);
     delete t;
-    return cuda_error(ctx, e, "cudaMemsetAsync(table)");
-  }
-  if (n) {
-    k_jb_build<<<grid_for(ctx, n, kThreads), kThreads, 0, s>>>(d_keys, d_payload, n,
-                                                                reinterpret_cast<JBucket *>(mem), t->rows,
-                                                                (uint32_t)(nbk - 1), t->meta, t->side,
-                                                                ctx->d_status);
-    rc = after_launch(ctx, "k_jb_build", s);
-    if (rc) {
-      pool_release(ctx, mem, s);
-      delete t;
-      return rc;
+    return code;
+  };
+  if (n && slots <= kSmallSlots) {
+    const size_t smem = slots * (with_pay ? 12 : 8);
+    cudaError_t e = cudaFuncSetAttribute(k_jb_build_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kSmallSlots * 12));
+    if (e != cudaSuccess) return fail(cuda_error(ctx, e, "k_jb_build_small"));
+    k_jb_build_small<<<1, kSmallThreads, smem, s>>>(d_keys, d_payload, (uint32_t)n, static_cast<uint4 *>(mem),
+                                                    reinterpret_cast<uint4 *>(t->rows), (uint32_t)slots, t->meta,
+                                                    t->side);
+    rc = after_launch(ctx, "k_jb_build_small", s);
+    if (rc) return fail(rc);
+  } else {
+    cudaError_t e = cudaMemsetAsync(mem, 0, clear_bytes, s);
+    if (e != cudaSuccess) return fail(cuda_error(ctx, e, "cudaMemsetAsync(table)"));
+    if (n) {
+      k_jb_build<<<grid_for(ctx, n, kThreads), kThreads, 0, s>>>(
+          d_keys, d_payload, n, static_cast<unsigned long long *>(mem), reinterpret_cast<int32_t *>(t->rows),
+          (uint32_t)(nbk - 1), t->meta, t->side, ctx->d_status);
+      rc = after_launch(ctx, "k_jb_build", s);
+      if (rc) return fail(rc);
     }
   }
   *out = t;
@@ -1201,7 +1251,7 @@ int gbj_reduce(gbj_ctx *ctx, const int32_t *d_col, const int32_t *d_rows,
   prof_mark(ctx, s);
   GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
   if (n == 0) return GBJ_OK;
-  k_reduce<<<grid_for(ctx, n, kThreads), kThreads, 0, s>>>(d_col, d_rows, n, spec, d_out);
+  launch_behind_init(k_reduce, grid_for(ctx, n, kThreads), kThreads, s, d_col, d_rows, n, spec, d_out);
   return after_launch(ctx, "k_reduce", s);
 }
 
