@@ -11,6 +11,8 @@
 // bytes, e.g. 2 MiB for 2^24 positions: L2-resident), set with atomicOr and
 // tested with one 32-bit load per probe row.  Which rows pass is exactly the
 // reference's.
+#include <algorithm>
+
 #include "compact.cuh"
 #include "gbj_internal.cuh"
 
@@ -33,11 +35,11 @@ __global__ void __launch_bounds__(256)
 }
 
 struct BloomPred {
-  const int32_t *keys;
+  const int32_t *col;
   const uint32_t *bits;
   uint32_t mask;
-  __device__ __forceinline__ bool operator()(uint64_t i) const {
-    const uint32_t p = (uint32_t)keys[i] & mask;
+  __device__ __forceinline__ bool test(int32_t key) const {
+    const uint32_t p = (uint32_t)key & mask;
     return (__ldg(bits + (p >> 5)) >> (p & 31)) & 1u;
   }
 };

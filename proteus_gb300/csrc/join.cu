@@ -13,13 +13,11 @@
 // {key, row + 1} slots in a static device array.
 // Semantics are the reference's: every build row is inserted (duplicates
 // allowed) and a probe row meets every build row with an equal key.
-#include <cooperative_groups.h>
+#include <algorithm>
 
 #include "compact.cuh"
 #include "gbj_internal.cuh"
-#include "scan.cuh"
 
-namespace cg = cooperative_groups;
 using namespace gbj;
 
 namespace {
@@ -427,59 +425,6 @@ __global__ void __launch_bounds__(kThreads, GBJ_JB_MIN_BLOCKS)
   gbjd::block_flush(spec, acc, red, out);
 }
 
-// Pair output over the bucketed table (warp-aggregated output reservations).
-template <bool kPay>
-__global__ void __launch_bounds__(kThreads)
-    k_jb_probe_pairs(const int32_t *__restrict__ keys, const int32_t *__restrict__ prows, uint64_t n,
-                     const JBucket *__restrict__ bk, const int4 *__restrict__ rows, uint32_t bmask,
-                     const uint32_t *__restrict__ meta, const int32_t *__restrict__ side,
-                     int32_t *__restrict__ out_b, int32_t *__restrict__ out_p, uint64_t cap,
-                     unsigned long long *count, uint32_t *status) {
-  const bool unique = meta[0] == 0;
-  const uint32_t nside = meta[1];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  auto emit = [&](int32_t br, int32_t pr) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(count, (unsigned long long)g.size());
-    base = g.shfl(base, 0) + g.thread_rank();
-    if (base < cap) {
-      out_b[base] = br;
-      out_p[base] = pr;
-    } else {
-      gbjd::latch(status, GBJ_DEV_CAPACITY);
-    }
-  };
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int32_t k = keys[i];
-    const int32_t pr = prows ? prows[i] : (int32_t)i;
-    const int32_t kf = k ^ kKeyFlip;
-    if (kf == 0) {
-      for (uint32_t s = 0; s < nside; ++s) {
-        emit(side[s], pr);
-      }
-      continue;
-    }
-    uint32_t b = gbjd::fmix32((uint32_t)k) & bmask;
-    for (uint32_t step = 0; step <= bmask; ++step) {
-      const JBucket e = ld_bucket(&bk[b]);
-      uint32_t hits = hits4(e.k, kf);
-      bool stop = room4(e.k);
-      while (hits) {
-        const uint32_t idx = __ffs(hits) - 1;
-        emit(lane4(kPay ? __ldg(&rows[b]) : e.x, idx) - 1, pr);
-        if (unique) {
-          stop = true;
-          break;
-        }
-        hits &= hits - 1;
-      }
-      if (stop) break;
-      b = (b + 1) & bmask;
-    }
-  }
-}
-
 // ------------------------------------------------ int64-key table
 // gbj_join_build_i64's table: 32-byte buckets of two slots -- two keys
 // (xor 2^63, so zero marks an empty slot; INT64_MIN goes to the side list),
@@ -553,7 +498,7 @@ __global__ void __launch_bounds__(kThreads)
   if (dup) meta[0] = 1;
 }
 
-// ------------------------------------------------ probe with any aggregate list
+// ------------------------------ probe with any aggregate list, or pair output
 // The two table layouts as k_jb_probe_list reads them.
 struct JTable {
   const void *bk;
@@ -611,11 +556,21 @@ constexpr int kListWarps = kListThreads / 32;
 // probes that go on past their home bucket (the last bucket looked at, and
 // how many are left; for the lowest key, which has no bucket, the next side
 // entry).
-template <typename Key>
+// Pair output: matches wait in a buffer of 256 {build row, probe row}.
+constexpr uint32_t kPairBuf = 256;
+
+template <typename Key, bool kPairs>
 struct ListQueue {
-  Key mkey[64];
-  uint64_t mprow[64];
-  int32_t mbv[64], mpv[64], mbr[64];
+  union {
+    struct {
+      Key mkey[64];
+      uint64_t mprow[64];
+      int32_t mbv[64], mpv[64], mbr[64];
+    };
+    struct {
+      int32_t pb[kPairs ? kPairBuf : 1], pp[kPairs ? kPairBuf : 1];
+    };
+  };
   Key wkey[64];
   uint64_t wprow[64];
   int32_t wpv[64];
@@ -637,29 +592,58 @@ struct ListQueue {
 // Measured on GB300, 1.5 M int64 build rows (two per key), 20 M probes, COUNT
 // + SUM + MIN + MAX: 8.21 ms before, 0.54 ms now (one row per key: 4.54 -> 0.23
 // ms; the same over int32 keys: 0.90 -> 0.22 ms).
+//
+// kMaxA = 0 is the pair output: `pay` holds the probe rows' ids (null: their
+// positions), matches wait in the warp's buffer, and one reservation in the
+// output takes 225 to 256 of them (one per 32 probes was 75 us of an atomic's
+// turn for 1.7 M probes, now 26 us).
+struct PairOut {
+  int32_t *build, *probe;
+  uint64_t cap;
+  unsigned long long *count;
+  uint32_t *status;
+};
+
 template <typename L, int kMaxA>
 __global__ void __launch_bounds__(kListThreads, kListCtas)
     k_jb_probe_list(const typename L::Key *__restrict__ keys, const int32_t *__restrict__ pay, uint64_t n,
-                    JTable t, gbj::AggSpec spec, int64_t *out) {
+                    JTable t, gbj::AggSpec spec, int64_t *out, PairOut po) {
   using Key = typename L::Key;
   using Bucket = typename L::Bucket;
-  __shared__ int64_t red[32 * GBJ_MAX_AGGS];
-  __shared__ ListQueue<Key> s_q[kListWarps];
+  constexpr bool kPairs = kMaxA == 0;
+  __shared__ int64_t red[kPairs ? 1 : 32 * GBJ_MAX_AGGS];
+  __shared__ ListQueue<Key, kPairs> s_q[kListWarps];
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  ListQueue<Key> &q = s_q[threadIdx.x >> 5];
+  ListQueue<Key, kPairs> &q = s_q[threadIdx.x >> 5];
   const bool unique = t.meta[0] == 0;
   const uint32_t nside = t.meta[1];
-  bool need_row = false;
+  bool need_row = kPairs;
 #pragma unroll
   for (int j = 0; j < kMaxA; ++j)
     if (j < spec.n)
       need_row |= spec.operand[j] == GBJ_VAL_BUILD_ROWID || spec.operand[j] == GBJ_VAL_ROWID_XOR;
-  int64_t v[kMaxA];
+  int64_t v[kPairs ? 1 : kMaxA];
 #pragma unroll
   for (int j = 0; j < kMaxA; ++j) v[j] = j < spec.n ? gbjd::agg_identity(spec.op[j]) : 0;
 
   uint32_t mn = 0, mh = 0;  // the ring's length and head (warp-uniform)
+  // writes the buffered pairs
+  auto flush = [&]() {
+    __syncwarp();
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(po.count, (unsigned long long)mn);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (uint32_t i = lane; i < mn; i += 32) {
+      if (base + i < po.cap) {
+        po.build[base + i] = q.pb[i];
+        po.probe[base + i] = q.pp[i];
+      }
+    }
+    if (base + mn > po.cap && lane == 0) gbjd::latch(po.status, GBJ_DEV_CAPACITY);
+    __syncwarp();
+    mn = 0;
+  };
   // applies the first `c` (<= 32) matches of the ring
   auto apply = [&](uint32_t c) {
     __syncwarp();
@@ -684,16 +668,27 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
       if (!bal) break;
       if (hits) {
         const uint32_t i = __ffs(hits) - 1;
-        const uint32_t p = (mh + mn + __popc(bal & lt)) & 63u;
-        q.mkey[p] = k;
-        q.mprow[p] = prow;
-        q.mpv[p] = pv;
-        q.mbv[p] = srow < 0 ? L::value(e, i) : t.bpay ? __ldg(t.bpay + srow) : 0;
-        q.mbr[p] = srow >= 0 ? srow : need_row ? L::row(t, e, b, i) : 0;
+        const int32_t br = srow >= 0 ? srow : need_row ? L::row(t, e, b, i) : 0;
+        if (kPairs) {
+          const uint32_t p = mn + __popc(bal & lt);
+          q.pb[p] = br;
+          q.pp[p] = pv;
+        } else {
+          const uint32_t p = (mh + mn + __popc(bal & lt)) & 63u;
+          q.mkey[p] = k;
+          q.mprow[p] = prow;
+          q.mpv[p] = pv;
+          q.mbv[p] = srow < 0 ? L::value(e, i) : t.bpay ? __ldg(t.bpay + srow) : 0;
+          q.mbr[p] = br;
+        }
         hits = unique ? 0u : hits & (hits - 1);
       }
       mn += __popc(bal);
-      if (mn >= 32) apply(32);
+      if (kPairs) {
+        if (mn > kPairBuf - 32) flush();
+      } else if (mn >= 32) {
+        apply(32);
+      }
     }
   };
   uint32_t wn = 0, wh = 0;  // the second ring's length and head
@@ -747,7 +742,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
   const uint64_t first = blockIdx.x * (uint64_t)kListThreads + (threadIdx.x & ~31u);  // of the warp
   auto load_key = [&](uint64_t i, Key &k, int32_t &p) {
     k = i < n ? __ldcs(keys + i) : 0;
-    p = pay && i < n ? __ldcs(pay + i) : 0;
+    p = pay ? (i < n ? __ldcs(pay + i) : 0) : kPairs ? (int32_t)i : 0;
   };
   Key k0, k1;
   int32_t p0, p1;
@@ -774,62 +769,21 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
     while (wn >= 32) walk(32);
   }
   while (wn) walk(wn < 32 ? wn : 32);
-  while (mn) apply(mn < 32 ? mn : 32);
-  gbjd::Acc acc;
+  if constexpr (kPairs) {
+    if (mn) flush();
+  } else {
+    while (mn) apply(mn < 32 ? mn : 32);
+    gbjd::Acc acc;
 #pragma unroll
-  for (int j = 0; j < GBJ_MAX_AGGS; ++j) acc.v[j] = j < kMaxA ? v[j < kMaxA ? j : 0] : 0;
-  gbjd::after_init();
-  gbjd::block_flush(spec, acc, red, out);
-}
-
-// Pair output over the int64-key table (warp-aggregated output reservations).
-__global__ void __launch_bounds__(kThreads)
-    k_jb64_probe_pairs(const int64_t *__restrict__ keys, const int32_t *__restrict__ prows, uint64_t n,
-                       const JBucket64 *__restrict__ bk, uint64_t bmask, const uint32_t *__restrict__ meta,
-                       const int32_t *__restrict__ side, int32_t *__restrict__ out_b,
-                       int32_t *__restrict__ out_p, uint64_t cap, unsigned long long *count, uint32_t *status) {
-  const bool unique = meta[0] == 0;
-  const uint32_t nside = meta[1];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  auto emit = [&](int32_t br, int32_t pr) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(count, (unsigned long long)g.size());
-    base = g.shfl(base, 0) + g.thread_rank();
-    if (base < cap) {
-      out_b[base] = br;
-      out_p[base] = pr;
-    } else {
-      gbjd::latch(status, GBJ_DEV_CAPACITY);
-    }
-  };
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int64_t k = keys[i];
-    const int32_t pr = prows ? prows[i] : (int32_t)i;
-    const unsigned long long kf = (unsigned long long)k ^ kFlip64;
-    if (kf == 0) {
-      for (uint32_t s = 0; s < nside; ++s) {
-        emit(side[s], pr);
-      }
-      continue;
-    }
-    uint64_t b = fmix64((uint64_t)k) & bmask;
-    for (uint64_t step = 0; step <= bmask; ++step) {
-      const JBucket64 e = ld_bucket64(&bk[b]);
-      bool stop = e.k[0] == 0 || e.k[1] == 0;
-      for (int j = 0; j < 2; ++j) {
-        if (e.k[j] == kf) {
-          emit(e.x[j].y - 1, pr);
-          if (unique) stop = true;
-        }
-      }
-      if (stop) break;
-      b = (b + 1) & bmask;
-    }
+    for (int j = 0; j < GBJ_MAX_AGGS; ++j) acc.v[j] = j < kMaxA ? v[j < kMaxA ? j : 0] : 0;
+    gbjd::after_init();
+    gbjd::block_flush(spec, acc, red, out);
   }
 }
 
-// Column reduce (Reduce over one column, optional row list).
+// Column reduce (Reduce over one column, optional row list): four rows of a
+// thread in flight.
+template <int kMaxA>
 __global__ void __launch_bounds__(kThreads)
     k_reduce(const int32_t *__restrict__ col, const int32_t *__restrict__ rows,
              uint64_t n, gbj::AggSpec spec, int64_t *out) {
@@ -837,31 +791,51 @@ __global__ void __launch_bounds__(kThreads)
   gbjd::Acc acc;
   acc.init(spec);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int64_t r = rows ? rows[i] : (int64_t)i;
-    const int64_t v = col ? col[r] : 0;
-    acc.update(spec, (int32_t)v, v, v, r, r);
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
+    int64_t r[4];
+    int32_t v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint64_t k = i + u * stride;
+      r[u] = rows ? (k < n ? __ldg(rows + k) : 0) : (int64_t)k;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = col && i + u * stride < n ? __ldg(col + r[u]) : 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i + u * stride < n) {
+#pragma unroll
+        for (int j = 0; j < kMaxA; ++j)
+          if (j < spec.n) gbjd::agg_step(acc.v[j], spec.op[j], spec.operand[j], v[u], v[u], v[u], r[u], r[u]);
+      }
+    }
   }
   gbjd::after_init();
   gbjd::block_flush(spec, acc, red, out);
 }
 
-__global__ void k_gather(const int32_t *__restrict__ col,
-                         const int32_t *__restrict__ rows, uint64_t n,
-                         int32_t *__restrict__ out) {
+// Four rows of a thread in flight.
+__global__ void __launch_bounds__(256)
+    k_gather(const int32_t *__restrict__ col, const int32_t *__restrict__ rows, uint64_t n,
+             int32_t *__restrict__ out) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-    out[i] = col[rows[i]];
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
+    int32_t r[4], v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) r[u] = i + u * stride < n ? __ldcs(rows + i + u * stride) : 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = i + u * stride < n ? __ldg(col + r[u]) : 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * stride < n) out[i + u * stride] = v[u];
+  }
 }
 
 // Range predicate of gbj_select_range (inclusive bounds).
 struct RangePred {
   const int32_t *col;
   int32_t lo, hi;
-  __device__ __forceinline__ bool operator()(uint64_t i) const {
-    const int32_t v = col[i];
-    return v >= lo && v <= hi;
-  }
+  __device__ __forceinline__ bool test(int32_t v) const { return v >= lo && v <= hi; }
 };
 
 int grid_for_sms(int sm_count, uint64_t work, int threads, int per_sm = 4) {
@@ -911,7 +885,15 @@ void launch_jb_list(int sm_count, const gbj_table *t, uint64_t nbk, const typena
   const JTable jt{t->slots, t->rows, (uint32_t)(nbk - 1), t->payload, t->meta, t->side};
   const int grid = grid_for_sms(sm_count, n, kListThreads, kListCtas);
   launch_behind_init(spec.n <= 4 ? k_jb_probe_list<L, 4> : k_jb_probe_list<L, 8>, grid, kListThreads, s, keys, pay, n,
-                     jt, spec, out);
+                     jt, spec, out, PairOut{});
+}
+
+template <typename L>
+void launch_jb_pairs(int sm_count, const gbj_table *t, uint64_t nbk, const typename L::Key *keys, const int32_t *prows,
+                     uint64_t n, const PairOut &po, cudaStream_t s) {
+  const JTable jt{t->slots, t->rows, (uint32_t)(nbk - 1), t->payload, t->meta, t->side};
+  k_jb_probe_list<L, 0><<<grid_for_sms(sm_count, n, kListThreads, kListCtas), kListThreads, 0, s>>>(
+      keys, prows, n, jt, gbj::AggSpec{}, nullptr, po);
 }
 
 // Probe kernel over a bucketed table: 16-byte probe loads when both probe
@@ -1134,16 +1116,10 @@ int gbj_join_probe_pairs(gbj_ctx *ctx, const gbj_table *t, const int32_t *d_keys
   prof_mark(ctx, s);
   GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
   if (n == 0) return GBJ_OK;
-  const JBucket *bk = static_cast<const JBucket *>(t->slots);
-  const uint32_t bmask = (uint32_t)((t->mask + 1) / 4 - 1);
-  if (t->rows)
-    k_jb_probe_pairs<true><<<grid_for(ctx, n, kThreads), kThreads, 0, s>>>(
-        d_keys, d_probe_rows, n, bk, t->rows, bmask, t->meta, t->side, d_build_rows, d_out_probe_rows, capacity,
-        (unsigned long long *)d_count, ctx->d_status);
-  else
-    k_jb_probe_pairs<false><<<grid_for(ctx, n, kThreads), kThreads, 0, s>>>(
-        d_keys, d_probe_rows, n, bk, nullptr, bmask, t->meta, t->side, d_build_rows, d_out_probe_rows, capacity,
-        (unsigned long long *)d_count, ctx->d_status);
+  const PairOut po{d_build_rows, d_out_probe_rows, capacity, (unsigned long long *)d_count, ctx->d_status};
+  const uint64_t nbk = (t->mask + 1) / 4;
+  if (t->rows) launch_jb_pairs<JLayout32<true>>(ctx->sm_count, t, nbk, d_keys, d_probe_rows, n, po, s);
+  else launch_jb_pairs<JLayout32<false>>(ctx->sm_count, t, nbk, d_keys, d_probe_rows, n, po, s);
   return after_launch(ctx, "k_jb_probe_pairs", s);
 }
 
@@ -1232,10 +1208,9 @@ int gbj_join_probe_pairs_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_
   prof_mark(ctx, s);
   GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(uint64_t), s));
   if (n == 0) return GBJ_OK;
-  k_jb64_probe_pairs<<<grid_for(ctx, n, kThreads), kThreads, 0, s>>>(
-      d_keys, d_probe_rows, n, static_cast<const JBucket64 *>(t->slots), (t->mask + 1) / 2 - 1, t->meta, t->side,
-      d_build_rows, d_out_probe_rows, capacity, (unsigned long long *)d_count, ctx->d_status);
-  return after_launch(ctx, "k_jb64_probe_pairs", s);
+  const PairOut po{d_build_rows, d_out_probe_rows, capacity, (unsigned long long *)d_count, ctx->d_status};
+  launch_jb_pairs<JLayout64>(ctx->sm_count, t, (t->mask + 1) / 2, d_keys, d_probe_rows, n, po, s);
+  return after_launch(ctx, "k_jb_probe_pairs", s);
 }
 
 int gbj_reduce(gbj_ctx *ctx, const int32_t *d_col, const int32_t *d_rows,
@@ -1251,7 +1226,8 @@ int gbj_reduce(gbj_ctx *ctx, const int32_t *d_col, const int32_t *d_rows,
   prof_mark(ctx, s);
   GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
   if (n == 0) return GBJ_OK;
-  launch_behind_init(k_reduce, grid_for(ctx, n, kThreads), kThreads, s, d_col, d_rows, n, spec, d_out);
+  launch_behind_init(spec.n <= 2 ? k_reduce<2> : k_reduce<GBJ_MAX_AGGS>, grid_for(ctx, n, kThreads), kThreads, s, d_col,
+                     d_rows, n, spec, d_out);
   return after_launch(ctx, "k_reduce", s);
 }
 
@@ -1357,8 +1333,3 @@ int gbj_join_agg_noalloc(const int32_t *d_build_keys, const int32_t *d_build_pay
 }
 
 }  // extern "C"
-
-// Shared by every ordered compaction (compact.cuh): the total row count.
-__global__ void gbj::k_compact_total(const uint64_t *off, uint64_t ntiles, uint64_t *dst) {
-  *dst = off[ntiles];
-}

@@ -1,16 +1,7 @@
-// Device-wide exclusive prefix sum over uint64 counters (multi-level,
-// stream-ordered), used for compaction; and the offsets of a small table
-// by one CTA, used by the partitioner and the partitioned operators.
+// Exclusive prefix sums by one CTA: the offsets of a small table, used by the
+// partitioner and the partitioned operators.
 #pragma once
 #include "gbj_internal.cuh"
-
-namespace gbj {
-
-// out[i] = sum(in[0..i)); out[n] = total (out must hold n + 1 entries).
-// `in` and `out` may alias.  Uses pool scratch for the block sums.
-int scan_u64(gbj_ctx *ctx, const uint64_t *in, uint64_t *out, uint64_t n,
-             cudaStream_t s);
-}  // namespace gbj
 
 namespace gbjd {
 
