@@ -391,11 +391,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     uint64_t lo, hi;
     bool whole = false;
     if (kPairs) {
-      uint32_t a = 0, b = P;
-      while (b - a > 1) {
-        const uint32_t mid = (a + b) >> 1;
-        if (item_off[mid] <= item) a = mid; else b = mid;
-      }
+      const uint32_t a = gbjd::item_partition(item_off, P, total_items, item);
       const uint64_t p0 = poff[a], p1 = poff[a + 1];
       lo = p0 + (item - item_off[a]) * w;
       hi = lo + w < p1 ? lo + w : p1;
@@ -611,8 +607,11 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
 
   if (strategy == 1) {
     GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
-    // raw input in items of w rows; level 1 persists for the CTA's lifetime
-    const uint64_t w = std::max<uint64_t>(1u << 16, (n + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8));
+    // raw input in items of w rows; level 1 persists for the CTA's lifetime.
+    // Eight items for each SM, but none shorter than 8192 rows: with 65,536
+    // the smaller inputs left most SMs idle (2^20 rows, 2000 groups 157 -> 63 us;
+    // 2^22 rows, 16 groups 74 -> 48 us; 2^24 rows and up unchanged)
+    const uint64_t w = std::max<uint64_t>(8192, (n + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8));
     const uint64_t wq = (w + 3) / 4 * 4;
     tslots_arg = (uint32_t)std::min<uint64_t>(kSlots, std::max<uint64_t>(64, next_pow2(16 * (hint ? hint : groups_cap))));
     pick_rlog();
@@ -620,14 +619,24 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
     if (aligned) GBJ_TRY(launch(k_groupby<false, true>, (int)tslots_arg, nullptr, wq, nullptr, nullptr, 0));
     else GBJ_TRY(launch(k_groupby<false, false>, (int)tslots_arg, nullptr, wq, nullptr, nullptr, 0));
   } else {
-    // partition so each partition holds ~kSlots/4 groups; add bits (without
-    // adding a partitioning pass) so partitions fit one work item of w rows
-    // and are emitted directly
-    const uint64_t w = 1u << 17;
+    // Partition so each partition holds ~kSlots/4 groups.  Then add bits,
+    // without adding a partitioning pass, until a partition has 16,384 rows
+    // (4 M rows, 5000 groups: 8 bits 121 us, 6 bits 147) and is usually one work
+    // item, which is emitted directly.  One pass over 9 to 11 bits costs less
+    // than over 12, so there the items are longer instead (2^28 rows, 2^20
+    // groups: 11 bits 2840 us, 12 bits 3032).  An item has a quarter of an SM's
+    // share of the rows, so that a skewed key's rows spread over the SMs, but no
+    // fewer than 32,768, which its merge into the global table must be worth
+    // (Zipf 1.0, against items of 131,072 rows: 2^22 rows in 100,000 groups
+    // 235 -> 117 us, 2^24 in 300,000 373 -> 266; uniform 2^24 in 100,000, where
+    // partitions are now two items, 212 -> 225).
     int bits = 1;
     while (bits < kMaxPartBits && (groups_cap >> bits) > (uint64_t)kSlots / 4) ++bits;
-    const int free_bits = bits <= 8 ? 8 : kMaxPartBits;
-    while (bits < free_bits && (n >> bits) > w / 2) ++bits;
+    const int free_bits = bits <= 8 ? 8 : bits <= 11 ? 11 : kMaxPartBits;
+    const uint64_t rows = bits <= 11 ? 16384 : 65536;
+    const uint64_t w = std::min<uint64_t>(bits > 8 && bits <= 11 ? 1u << 18 : 1u << 17,
+                                          std::max<uint64_t>(32768, next_pow2(n / (4 * ctx->sm_count))));
+    while (bits < free_bits && (n >> bits) > rows) ++bits;
     if (params && params->hash_bits > 0 && strategy == 2 && !hint)
       bits = std::min(params->hash_bits, kMaxPartBits);
     if (tuned_bits > 0) bits = std::min<int>(tuned_bits, kMaxPartBits);

@@ -577,40 +577,6 @@ __global__ void __launch_bounds__(1024)
   }, items, s_scan);
 }
 
-// Partition of work item `item`: largest p with item_off[p] <= item, where
-// item_off[0] = 0 <= item < item_off[P] = total.  Starts from the
-// proportional guess and gallops, so the common case (about one item per
-// partition) costs two or three dependent loads.
-__device__ __forceinline__ uint32_t item_partition(const uint64_t *__restrict__ off, uint32_t P,
-                                                   uint64_t total, uint64_t item) {
-  uint32_t lo = (uint32_t)((item * (uint64_t)P) / total);
-  if (lo >= P) lo = P - 1;
-  uint32_t hi;
-  if (off[lo] <= item) {
-    uint32_t step = 1;
-    hi = lo + 1;
-    while (hi < P && off[hi] <= item) {
-      lo = hi;
-      step <<= 1;
-      hi = lo + step < P ? lo + step : P;
-    }
-  } else {
-    uint32_t step = 1;
-    hi = lo;
-    for (;;) {  // off[hi] > item; off[0] = 0 <= item ends the walk
-      lo = hi > step ? hi - step : 0;
-      if (off[lo] <= item) break;
-      hi = lo;
-      step <<= 1;
-    }
-  }
-  while (hi - lo > 1) {  // off[lo] <= item < off[hi]
-    const uint32_t mid = (lo + hi) >> 1;
-    if (off[mid] <= item) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
 // kAggRows: both sides carry row positions; a match first compares the
 // minor keys (when given), then reads the payloads by row.
 enum : int { kAggList = 0, kAggCountXor = 1, kAggCountProduct = 2, kAggRows = 3 };
@@ -715,7 +681,7 @@ __global__ void __launch_bounds__(kThreads, kCtas)
     const unsigned long long item = atomicAdd(item_ctr, 1ull);
     s_it.valid = item < total;
     if (item < total) {
-      const uint32_t p = item_partition(item_off, P, total, item);
+      const uint32_t p = gbjd::item_partition(item_off, P, total, item);
       const uint64_t r0 = ro[p], r1 = ro[p + 1], s0 = so[p], s1 = so[p + 1];
       const uint64_t nrc = (r1 - r0 + kRMax - 1) / kRMax;
       const uint64_t local = item - item_off[p];

@@ -22,3 +22,41 @@ int partition_tuples(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals,
                      bool hash_out = false);
 
 }  // namespace gbj
+
+namespace gbjd {
+
+// Partition of work item `item`: largest p with item_off[p] <= item, where
+// item_off[0] = 0 <= item < item_off[P] = total.  Starts from the
+// proportional guess and gallops, so the common case (about one item per
+// partition) costs two or three dependent loads.
+__device__ __forceinline__ uint32_t item_partition(const uint64_t *__restrict__ off, uint32_t P,
+                                                   uint64_t total, uint64_t item) {
+  uint32_t lo = (uint32_t)((item * (uint64_t)P) / total);
+  if (lo >= P) lo = P - 1;
+  uint32_t hi;
+  if (off[lo] <= item) {
+    uint32_t step = 1;
+    hi = lo + 1;
+    while (hi < P && off[hi] <= item) {
+      lo = hi;
+      step <<= 1;
+      hi = lo + step < P ? lo + step : P;
+    }
+  } else {
+    uint32_t step = 1;
+    hi = lo;
+    for (;;) {  // off[hi] > item; off[0] = 0 <= item ends the walk
+      lo = hi > step ? hi - step : 0;
+      if (off[lo] <= item) break;
+      hi = lo;
+      step <<= 1;
+    }
+  }
+  while (hi - lo > 1) {  // off[lo] <= item < off[hi]
+    const uint32_t mid = (lo + hi) >> 1;
+    if (off[mid] <= item) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+}  // namespace gbjd

