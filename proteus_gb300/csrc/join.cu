@@ -425,6 +425,193 @@ __global__ void __launch_bounds__(kThreads, GBJ_JB_MIN_BLOCKS)
   gbjd::block_flush(spec, acc, red, out);
 }
 
+// Probes whose home bucket does not end them: they look at their next bucket
+// 32 at a time.
+template <typename X>
+struct WalkRing {
+  int32_t kf[128];
+  uint32_t b[128];  // the next bucket to look at
+  X x[128];         // the probe's payload (product list) or row (xor list)
+};
+
+// The same for a table that is more than a third full, where a tenth of the
+// probes and more go on to the next bucket.  Taken where the need is found,
+// those walks leave 20 of 32 lanes active; here they wait in the warp's ring
+// and 32 of them look at their next bucket together.  Four probes a lane are in
+// flight as above, in tiles of 128 a warp.  Bound by the buckets' way from L2
+// and by issue.  Measured on GB300, 2^24 probes, walks alone / ring, us: 2^20
+// dense keys 102 / 84, 2^20 keys without a pattern and half the probes without a
+// match 132 / 93, two rows a key 290 / 166, three and the xor list 459 / 207.
+// In a table that is less full its instructions and its shared memory, which
+// the first-level cache then lacks, only cost (2^26 probes: 5000 rows,
+// load 0.3, 199 / 248; 20,000 rows, 0.31, 270 / 274; 60,000 rows, 0.46, 333 /
+// 287).
+template <bool kVec, int kAgg, bool kPay>
+__global__ void __launch_bounds__(kThreads, GBJ_JB_MIN_BLOCKS)
+    k_jb_probe_ring(const int32_t *__restrict__ keys, const int32_t *__restrict__ pay, uint64_t n,
+                    const JBucket *__restrict__ bk, const int4 *__restrict__ rows, uint32_t bmask,
+                    const int32_t *__restrict__ bpay, const uint32_t *__restrict__ meta,
+                    const int32_t *__restrict__ side, gbj::AggSpec spec, int64_t *out) {
+  __shared__ int64_t red[32 * GBJ_MAX_AGGS];
+  using X = std::conditional_t<kAgg == kAggCountProduct, int32_t, int64_t>;
+  __shared__ WalkRing<X> s_ring[kThreads / 32];
+  static_assert(kAgg != kAggGeneric, "other aggregate lists: k_jb_probe_list");
+  constexpr int G = kJbGroup;  // probes per lane at a time
+  static_assert(G == 4, "one 16-byte load a lane");
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  WalkRing<X> &ring = s_ring[threadIdx.x >> 5];
+  int64_t a_cnt = 0, a_sum = 0;
+  const bool unique = meta[0] == 0;
+  const uint32_t nside = meta[1];
+  // folds the matching slots of bucket b (contents e) into the aggregate;
+  // returns the number of matches
+  auto visit = [&](int32_t kf, X x, uint32_t b, const JBucket &e) -> uint32_t {
+    const bool m0 = e.k.x == kf, m1 = e.k.y == kf, m2 = e.k.z == kf, m3 = e.k.w == kf;
+    const uint32_t c = (uint32_t)m0 + (uint32_t)m1 + (uint32_t)m2 + (uint32_t)m3;
+    a_cnt += c;
+    if (kAgg == kAggCountProduct) {
+      if (kPay)
+        a_sum += ((int64_t)(m0 ? e.x.x : 0) + (m1 ? e.x.y : 0) + (int64_t)(m2 ? e.x.z : 0) + (m3 ? e.x.w : 0)) * x;
+    } else if (c) {
+      const int4 rw = kPay ? __ldg(&rows[b]) : e.x;
+      a_sum += (m0 ? ((int64_t)(rw.x - 1) ^ x) : 0) + (m1 ? ((int64_t)(rw.y - 1) ^ x) : 0) +
+               (m2 ? ((int64_t)(rw.z - 1) ^ x) : 0) + (m3 ? ((int64_t)(rw.w - 1) ^ x) : 0);
+    }
+    return c;
+  };
+  // a probe key INT32_MIN meets the side list
+  auto side_probe = [&](X x) {
+    for (uint32_t s = 0; s < nside; ++s) {
+      const int32_t r = side[s];
+      a_cnt += 1;
+      if (kAgg == kAggCountProduct) a_sum += (kPay ? (int64_t)bpay[r] : 0) * x;
+      else a_sum += (int64_t)r ^ x;
+    }
+  };
+  uint32_t qn = 0, qh = 0;  // the ring's length and head (warp-uniform)
+  auto push = [&](bool yes, int32_t kf, X x, auto b) {
+    const unsigned bal = __ballot_sync(0xffffffffu, yes);
+    if (bal == 0) return;
+    if (yes) {
+      const uint32_t p = (qh + qn + __popc(bal & lt)) & 127u;
+      ring.kf[p] = kf;
+      ring.b[p] = b();
+      ring.x[p] = x;
+    }
+    qn += __popc(bal);
+  };
+  auto home = [&](int32_t kf) { return gbjd::fmix32((uint32_t)(kf ^ kKeyFlip)) & bmask; };
+  // the next bucket of the first c (<= 32) probes of the ring.  With unique
+  // keys those have no match yet, with others a match does not end them; the
+  // table is at most half full, and all of it is the most they look at.
+  auto walk = [&](uint32_t c) {
+    __syncwarp();
+    const bool mine = (uint32_t)lane < c;
+    const uint32_t p = (qh + lane) & 127u;
+    const int32_t kf = mine ? ring.kf[p] : 0;
+    const uint32_t b = mine ? ring.b[p] : 0, next = (b + 1) & bmask;
+    const X x = mine ? ring.x[p] : 0;
+    __syncwarp();  // read before any of them is written again
+    qh = (qh + c) & 127u;
+    qn -= c;
+    bool on = false;
+    if (mine) {
+      const JBucket e = ld_bucket(&bk[b]);
+      const uint32_t m = visit(kf, x, b, e);
+      on = !room4(e.k) && !(unique && m) && next != home(kf);
+    }
+    __syncwarp();
+    push(on, kf, x, [&] { return next; });
+  };
+  // a probe meets its home bucket (its contents in e): true when it goes on
+  auto meet = [&](int32_t k, X x, const JBucket &e) -> bool {
+    const int32_t kf = k ^ kKeyFlip;
+    if (kf == 0) {
+      side_probe(x);
+      return false;
+    }
+    // the home bucket again where it is wanted: kept, it takes four registers
+    const uint32_t c = visit(kf, x, kPay && kAgg == kAggCountXor ? home(kf) : 0u, e);
+    return !room4(e.k) && !(unique && c);
+  };
+  auto enqueue = [&](bool on, int32_t k, X x) {
+    const int32_t kf = k ^ kKeyFlip;
+    push(on, kf, x, [&] { return (home(kf) + 1) & bmask; });
+  };
+  // tiles of 32 G probes; probe j of a lane is one of four neighbours, or with
+  // a column that is not 16-byte aligned one of every 32nd
+  constexpr uint32_t kTile = 32 * G;
+  constexpr bool kValues = kAgg == kAggCountProduct && kPay;
+  const bool values = kValues && pay;
+  const uint64_t tiles = n / kTile, stride = (uint64_t)gridDim.x * (kThreads / 32);
+  auto load = [&](const int32_t *col, uint64_t t, int32_t *v) {
+    if (kVec) {
+      const int4 v4 = __ldcs(reinterpret_cast<const int4 *>(col + t * kTile) + lane);
+      v[0] = v4.x, v[1] = v4.y, v[2] = v4.z, v[3] = v4.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < G; ++j) v[j] = __ldcs(col + t * kTile + j * 32 + lane);
+    }
+  };
+  uint64_t t = blockIdx.x * (uint64_t)(kThreads / 32) + (threadIdx.x >> 5);
+  int32_t nk[G], np[G] = {0, 0, 0, 0};
+  if (t < tiles) {
+    load(keys, t, nk);
+    if (values) load(pay, t, np);
+  }
+  for (; t < tiles; t += stride) {
+    int32_t kk[G], pp[G];
+    JBucket e[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      kk[j] = nk[j];
+      pp[j] = np[j];
+      e[j] = ld_bucket(&bk[gbjd::fmix32((uint32_t)kk[j]) & bmask]);
+    }
+    if (t + stride < tiles) {
+      load(keys, t + stride, nk);
+      if (values) load(pay, t + stride, np);
+    }
+    auto value = [&](int j) {
+      return kAgg == kAggCountProduct ? (X)pp[j] : (X)(t * kTile + (kVec ? lane * G + j : j * 32 + lane));
+    };
+    bool on[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j) on[j] = meet(kk[j], value(j), e[j]);
+    if (!__any_sync(0xffffffffu, on[0] | on[1] | on[2] | on[3])) continue;
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      enqueue(on[j], kk[j], value(j));
+      if (j & 1)
+        while (qn >= 32) walk(32);
+    }
+  }
+  if (t == tiles) {  // the last n mod 32 G probes: this warp's
+    for (uint64_t base = tiles * kTile; base < n; base += 32) {
+      const uint64_t i = base + lane;
+      bool on = false;
+      int32_t k = 0;
+      X x = 0;
+      if (i < n) {
+        k = keys[i];
+        x = kAgg == kAggCountProduct ? (X)(values ? pay[i] : 0) : (X)i;
+        on = meet(k, x, ld_bucket(&bk[gbjd::fmix32((uint32_t)k) & bmask]));
+      }
+      __syncwarp();
+      enqueue(on, k, x);
+      while (qn >= 32) walk(32);
+    }
+  }
+  while (qn) walk(qn < 32 ? qn : 32);
+  gbjd::Acc acc;
+  acc.init(spec);
+  acc.v[0] = a_cnt;
+  acc.v[1] = a_sum;
+  gbjd::after_init();
+  gbjd::block_flush(spec, acc, red, out);
+}
+
 // ------------------------------------------------ int64-key table
 // gbj_join_build_i64's table: 32-byte buckets of two slots -- two keys
 // (xor 2^63, so zero marks an empty slot; INT64_MIN goes to the side list),
@@ -692,7 +879,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas)
     }
   };
   uint32_t wn = 0, wh = 0;  // the second ring's length and head
-  auto queue_walk = [&](bool go_on, Key k, int32_t pv, uint64_t prow, uint32_t b, uint32_t left) {
+  auto queue_walk = [&](bool go_on, Key k, int32_t pv, uint64_t prow, auto b, uint32_t left) {
     const unsigned bal = __ballot_sync(0xffffffffu, go_on);
     if (go_on) {
       const uint32_t p = (wh + wn + __popc(bal & lt)) & 63u;
@@ -913,9 +1100,10 @@ void launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, co
   }
   const int gv = grid_for_sms(sm_count, (n + kJbGroup - 1) / kJbGroup, kThreads, 2);
   const int gs = grid_for_sms(sm_count, n, kThreads);
-#define GBJ_JB_PROBE(V, A)                                                                                  \
-  launch_behind_init(k_jb_probe_agg<V, A, kPay>, V ? gv : gs, kThreads, s, keys, pay, n, bk, t->rows, bmask, \
-                     t->payload, t->meta, t->side, spec, out)
+  const bool ring = 3 * t->n > t->mask + 1;  // the table is more than a third full: times at k_jb_probe_ring
+#define GBJ_JB_PROBE(V, A)                                                                                   \
+  launch_behind_init(ring ? k_jb_probe_ring<V, A, kPay> : k_jb_probe_agg<V, A, kPay>, V || ring ? gv : gs, kThreads, \
+                     s, keys, pay, n, bk, t->rows, bmask, t->payload, t->meta, t->side, spec, out)
   if (vec) {
     if (is_xor) GBJ_JB_PROBE(true, kAggCountXor);
     else GBJ_JB_PROBE(true, kAggCountProduct);
