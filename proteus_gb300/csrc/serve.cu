@@ -165,6 +165,11 @@ __device__ __forceinline__ int64_t g_claim(const SQ &q, int32_t g) {
   return -1;
 }
 
+// A table is sectors of four slots (32 bytes); tmask is its slots - 1.
+__device__ __forceinline__ uint32_t home_sector(uint32_t hash, uint64_t tmask) {
+  return hash & (uint32_t)(tmask >> 2);
+}
+
 // Build: each row's group is resolved to its group-table slot here, once,
 // and the join table stores {key | slot << 32}; a probe match then adds to
 // a known slot with no further lookup.
@@ -217,14 +222,18 @@ __global__ void __launch_bounds__(kThreads) k_serve_build(const SBatch *__restri
         continue;
       }
       const unsigned long long e = (unsigned long long)(uint32_t)k | ((unsigned long long)gs << 32);
-      uint64_t h = gbjd::fmix32((uint32_t)k) & q.tmask;
+      // the slots of the home sector from one that other hash bits choose, then
+      // of the following sectors
+      const uint32_t hash = gbjd::fmix32((uint32_t)k);
+      uint64_t h = home_sector(hash, q.tmask) * 4 + (hash >> 30);
       bool placed = false;
       for (uint64_t step = 0; step <= q.tmask; ++step) {
         if (atomicCAS(&q.table[h], kEmptySlot, e) == kEmptySlot) {
           placed = true;
           break;
         }
-        h = (h + 1) & q.tmask;
+        h = (h & ~3ull) | ((h + 1) & 3);
+        if ((step & 3) == 3) h = (h + 4) & q.tmask;
       }
       if (!placed) gbjd::latch(&slot->status[qi], GBJ_DEV_CAPACITY);
     }
@@ -241,14 +250,19 @@ __global__ void __launch_bounds__(kThreads) k_serve_build(const SBatch *__restri
 // of a slot in an item; later matches (duplicate-heavy builds) add their value
 // to the global 64-bit sum directly.
 //
-// A probe reads the 32-byte sector of its home slot (four slots in one load)
-// and goes on to the next sector only when no slot from its home on is empty;
-// those probes wait in the warp's ring and 32 of them take a sector each.
-// What bounds it is the latency of the table's sectors, in L2 or HBM: slot by
+// A table is sectors of four slots (32 bytes, one load).  A row takes a free
+// slot of its home sector or else of the next sectors, so a probe folds every
+// match among the four and goes on only when none of them is empty; those
+// probes wait in the warp's ring and 32 of them take a sector each.  Slot by
 // slot, where it was found, each probe of a warp waited for the longest of 32
-// chains.  The next probe's sector is loaded while this one's is looked at,
-// and its key one step earlier.  Measured on GB300, 24 queries of the serving
-// mix, 335 M probes in the large ones: 5.49 ms before, 3.60 ms now.
+// chains; slots taken in order from the home slot on sent twice as many probes
+// to the next sector.  The next probe's sector is loaded while this one's is
+// looked at, and its key one step earlier.  Bound by issue (58 % of it with
+// slots in order, 250 instructions for 32 probes) and by the sectors' latency;
+// two or three sectors a lane in flight, or smaller CTAs, were slower (5.4, 5.9,
+// 6.2 ms a batch against 5.1).  Measured on GB300, 24 queries of the serving
+// mix, 332 M probes in the large ones: 5.49 ms slot by slot, 3.60 ms in order of
+// the slots, 3.27 ms now.
 constexpr uint32_t kL1Exact = 65535;
 
 struct ServeQueue {
@@ -320,33 +334,37 @@ __global__ void __launch_bounds__(kProbeThreads, 2) k_serve_probe(const SBatch *
         }
       }
     };
-    // the matches among a sector's slots from `start` on; true: all of those are taken
-    auto visit = [&](bool ok, int32_t k, int32_t v, const Sector &e, uint32_t start) -> bool {
-      uint32_t eq = 0, empty = 0;
+    // the matches in a sector; true: all of its slots are taken
+    auto visit = [&](bool ok, int32_t k, int32_t v, const Sector &e) -> bool {
+      bool m[4], empty = false;
+      uint32_t gs = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        eq |= (uint32_t)((uint32_t)e.s[j] == (uint32_t)k) << j;
-        empty |= (uint32_t)((uint32_t)e.s[j] == kFlip) << j;
+      for (int j = 3; j >= 0; --j) {
+        m[j] = ok & ((int32_t)(uint32_t)e.s[j] == k);
+        empty |= (uint32_t)e.s[j] == kFlip;
+        if (m[j]) gs = (uint32_t)(e.s[j] >> 32);
       }
-      empty &= 0xfu << start;
-      // slots [start, first empty one)
-      uint32_t hits = ok ? eq & (0xfu << start) & (empty ? (empty & (0u - empty)) - 1u : 0xfu) : 0u;
-      while (__any_sync(0xffffffffu, hits != 0)) {
-        const int j = hits ? __ffs(hits) - 1 : 0;
-        const unsigned long long x = j == 0 ? e.s[0] : j == 1 ? e.s[1] : j == 2 ? e.s[2] : e.s[3];
-        add(hits != 0, (uint32_t)(x >> 32), v);
-        hits &= hits - 1;
+      add(m[0] | m[1] | m[2] | m[3], gs, v);
+      // a second match: equal build keys
+      if (__any_sync(0xffffffffu, (m[0] & (m[1] | m[2] | m[3])) | (m[1] & (m[2] | m[3])) | (m[2] & m[3]))) {
+        bool before = m[0];
+#pragma unroll
+        for (int j = 1; j < 4; ++j) {
+          add(before & m[j], (uint32_t)(e.s[j] >> 32), v);
+          before |= m[j];
+        }
       }
-      return ok && !empty;
+      return ok & !empty;
     };
     uint32_t qn = 0, qh = 0;  // the ring's length and head (warp-uniform)
-    auto push = [&](bool yes, int32_t k, int32_t v, uint32_t sec) {
+    auto push = [&](bool yes, int32_t k, int32_t v, auto sec) {
       const unsigned bal = __ballot_sync(0xffffffffu, yes);
+      if (bal == 0) return;
       if (yes) {
         const uint32_t p = (qh + qn + __popc(bal & lt)) & 63u;
         wq.k[p] = k;
         wq.v[p] = v;
-        wq.sec[p] = sec;
+        wq.sec[p] = sec();
       }
       qn += __popc(bal);
     };
@@ -361,46 +379,48 @@ __global__ void __launch_bounds__(kProbeThreads, 2) k_serve_probe(const SBatch *
       __syncwarp();  // read before any of them is written again
       qh = (qh + c) & 63u;
       qn -= c;
-      push(visit(mine, k, v, ld_sector(table, sec), 0), k, v, (sec + 1) & smask);
+      push(visit(mine, k, v, ld_sector(table, sec)), k, v, [&] { return (sec + 1) & smask; });
     };
-    auto load = [&](uint64_t i, int32_t &k, int32_t &v) {
-      k = i < hi ? __ldcs(pk + i) : 0;
-      v = i < hi ? __ldcs(pv + i) : 0;
+    // an item has at most 2^16 probes: 32-bit places in it
+    const int32_t *ik = pk + lo, *iv = pv + lo;
+    const uint32_t rows = (uint32_t)(hi - lo);
+    auto load = [&](uint32_t i, int32_t &k, int32_t &v) {
+      k = i < rows ? __ldcs(ik + i) : 0;
+      v = i < rows ? __ldcs(iv + i) : 0;
     };
-    const uint64_t first = lo + (threadIdx.x & ~31u);  // of the warp
+    auto home = [&](int32_t k) { return home_sector(gbjd::fmix32((uint32_t)k), tmask); };
     int32_t k0, v0, k1, v1;
-    load(first + lane, k0, v0);
-    uint32_t h0 = gbjd::fmix32((uint32_t)k0) & tmask;
-    Sector e0 = ld_sector(table, h0 >> 2);
-    load(first + kProbeThreads + lane, k1, v1);
-    for (uint64_t base = first; base < hi; base += kProbeThreads) {
+    load(threadIdx.x, k0, v0);
+    Sector e0 = ld_sector(table, home(k0));
+    load(threadIdx.x + kProbeThreads, k1, v1);
+    for (uint32_t base = threadIdx.x & ~31u; base < rows; base += kProbeThreads) {
       const int32_t k = k0, v = v0;
-      const uint32_t h = h0;
       const Sector e = e0;
       k0 = k1;
       v0 = v1;
-      h0 = gbjd::fmix32((uint32_t)k0) & tmask;
-      e0 = ld_sector(table, h0 >> 2);
-      load(base + 2 * kProbeThreads + lane, k1, v1);
-      const bool ok = base + lane < hi, to_side = k == INT32_MIN;
-      push(visit(ok && !to_side, k, v, e, h & 3u), k, v, ((h >> 2) + 1) & smask);
-      if (__any_sync(0xffffffffu, ok && to_side && side_n != 0))
-        for (unsigned long long j = 0; j < side_n; ++j) add(ok && to_side, (uint32_t)side[j], v);
+      e0 = ld_sector(table, home(k0));
+      load(base + lane + 2 * kProbeThreads, k1, v1);
+      const bool in = base + lane < rows, to_side = k == INT32_MIN;
+      const bool on = visit(in & !to_side, k, v, e);
+      push(on, k, v, [&] { return (home(k) + 1) & smask; });
+      if (__any_sync(0xffffffffu, in & to_side & (side_n != 0)))
+        for (unsigned long long j = 0; j < side_n; ++j) add(in & to_side, (uint32_t)side[j], v);
       while (qn >= 32) walk(32);
     }
     while (qn) walk(qn < 32 ? qn : 32);
     if (use_l1) {
       __syncthreads();
       // two lanes a slot: one adds the count, the other the sum
-      for (uint64_t i2 = threadIdx.x; i2 < 2 * (gmask + 2); i2 += blockDim.x) {
+      for (uint64_t w2 = threadIdx.x & ~31u; w2 < 2 * (gmask + 2); w2 += blockDim.x) {
+        const uint64_t i2 = w2 + lane;
         const uint32_t i = (uint32_t)(i2 >> 1);
-        const uint32_t c = l1_cnt[i];
+        const uint32_t c = i2 < 2 * (gmask + 2) ? l1_cnt[i] : 0;
         if (c) {
           const uint64_t in_ab = c < kL1Exact ? c : kL1Exact;  // matches summed in a / b
           const int64_t sum = (int64_t)(((uint64_t)l1_b[i] << 16) + l1_a[i]) - (int64_t)in_ab * (int64_t)kFlip;
           atomicAdd(&gacc[i2], i2 & 1 ? (unsigned long long)sum : (unsigned long long)c);
         }
-        __syncwarp(__activemask());
+        __syncwarp();
         if (c && !(i2 & 1)) {
           l1_cnt[i] = 0;
           l1_a[i] = 0;
