@@ -114,19 +114,25 @@ __device__ __forceinline__ void emit(const Out &o, uint64_t pos, int32_t key, ui
 //   key[]  key' (0 = empty)
 //   ext[]  {min', max'}: also the hints that decide whether a min/max
 //          atomic is issued
-//   cnt[]  rows
-//   a[], b[]  with u = value + 2^31 (unsigned, < 2^32), a sums the low 16
-//          bits of u and b the high 16 bits, so
-//          SUM(value) = b * 2^16 + a - count * 2^31.
-// a, b and cnt stay exact while a slot takes at most 65535 rows between
-// flushes; the kernel tracks a CTA-wide bound on every slot's count and moves
-// slots above kHot rows to level 2 before the bound could pass 65535.
-// cnt, a and b have 2^rlog columns per slot, column = lane mod 2^rlog: a
-// shared atomic costs a data-pipe pass per bank it hits twice, and with
-// lane-indexed columns the lanes of a warp that land on slots in one bank
-// fall on different banks (32 columns: never two lanes on one bank).  The
-// host takes as many columns as shared memory allows; a slot's value is the
-// sum of its columns.
+//   lo[], hi[]  with u = value + 2^31 (unsigned, < 2^32), lo sums u modulo
+//          2^32; hi counts lo's carries in its low 16 bits and the rows in its
+//          high 16 bits, so SUM(value) = carries * 2^32 + lo - rows * 2^31.
+// hi stays exact while a slot takes at most 65535 rows between flushes; the
+// kernel tracks a CTA-wide bound on every slot's count and moves slots above
+// kHot rows to level 2 before the bound could pass 65535.
+// lo and hi have 2^rlog columns per slot, column = lane mod 2^rlog: a shared
+// atomic costs a data-pipe pass per bank it hits twice, and with lane-indexed
+// columns the lanes of a warp that land on slots in one bank fall on different
+// banks.  The host takes as many columns as shared memory allows, but at most
+// 16: with 32 the columns of 32 slots that a warp clears or flushes together
+// are in one bank (2^20 rows, 16 groups: 62 us against 32).  A slot's value is
+// the sum of its columns.
+// The data pipe bounds the kernel, so what counts is a row's atomics: lo's
+// carry is seen from the value that its add returns, which leaves two for what
+// took three when count, low and high halves were summed apart.  Measured on
+// GB300, 2^28 rows, three / two: 16 groups 638 / 594 us, 64 groups 884 / 747,
+// 1000 groups 1006 / 909, 2^24 groups in partitions 1567 / 1447; adding four
+// rows' lo together before their hi was slower (16 groups 901).
 __device__ __forceinline__ uint32_t s_ld(uint32_t a) {
   uint32_t r;
   asm("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a));
@@ -146,51 +152,56 @@ __device__ __forceinline__ void s_st2(uint32_t a, uint2 v) {
 
 // The table's arrays by their shared-state-space addresses (32-bit).
 struct L1 {
-  uint32_t ext, key, cnt, a, b;
+  uint32_t ext, key, lo, hi;
   uint32_t mask;   // slots - 1
   uint32_t shift;  // 32 - log2(slots): the home slot is the hash's top bits
-  uint32_t rlog;   // log2 of the columns of cnt, a, b
+  uint32_t rlog;   // log2 of the columns of lo, hi
 
   // Lays the arrays out from shared address `base` for `slots` slots.
   __device__ __forceinline__ void place(uint32_t base, uint32_t slots, uint32_t rlog_) {
     rlog = rlog_;
     ext = base;
     key = ext + 8u * slots;
-    cnt = key + 4u * slots;
-    a = cnt + (4u * slots << rlog);
-    b = a + (4u * slots << rlog);
+    lo = key + 4u * slots;
+    hi = lo + (4u * slots << rlog);
     mask = slots - 1;
     shift = 32u - (uint32_t)__popc(slots - 1);
   }
-  // this lane's column of slot h (byte offset into cnt / a / b)
+  // this lane's column of slot h (byte offset into lo / hi)
   __device__ __forceinline__ uint32_t col(uint32_t h) const {
     return ((h << rlog) + ((threadIdx.x & 31) & ((1u << rlog) - 1))) * 4u;
   }
-  __device__ __forceinline__ uint32_t sum_cols(uint32_t arr, int i) const {
-    uint32_t v = 0;
-    for (uint32_t r = 0; r < (1u << rlog); ++r) v += s_ld(arr + (((uint32_t)i << rlog) + r) * 4u);
-    return v;
-  }
-  // a slot as {key', min', max', count} and {a, b} (block-synchronised paths)
+  // a slot as {key', min', max', count} and its biased sum (block-synchronised
+  // paths)
   __device__ __forceinline__ uint4 meta(int i) const {
     const uint2 e = s_ld2(ext + 8u * i);
     return make_uint4(s_ld(key + 4u * i), e.x, e.y, count(i));
   }
-  __device__ __forceinline__ uint2 sums(int i) const { return make_uint2(sum_cols(a, i), sum_cols(b, i)); }
-  __device__ __forceinline__ uint32_t count(int i) const { return sum_cols(cnt, i); }
+  __device__ __forceinline__ uint64_t sum(int i) const {
+    uint64_t v = 0;
+    for (uint32_t r = 0; r < (1u << rlog); ++r) {
+      const uint32_t o = (((uint32_t)i << rlog) + r) * 4u;
+      v += ((uint64_t)(s_ld(hi + o) & 0xffffu) << 32) + s_ld(lo + o);
+    }
+    return v;
+  }
+  __device__ __forceinline__ uint32_t count(int i) const {
+    uint32_t v = 0;
+    for (uint32_t r = 0; r < (1u << rlog); ++r) v += s_ld(hi + (((uint32_t)i << rlog) + r) * 4u) >> 16;
+    return v;
+  }
   __device__ __forceinline__ void reset(int i, uint32_t k) const {
     s_st(key + 4u * i, k);
     s_st2(ext + 8u * i, make_uint2(0, 0));
     for (uint32_t r = 0; r < (1u << rlog); ++r) {
       const uint32_t o = (((uint32_t)i << rlog) + r) * 4u;
-      s_st(cnt + o, 0);
-      s_st(a + o, 0);
-      s_st(b + o, 0);
+      s_st(lo + o, 0);
+      s_st(hi + o, 0);
     }
   }
 };
 // shared bytes per slot with 2^rlog accumulator columns
-__host__ __device__ constexpr size_t slot_bytes(int rlog) { return 12 + ((size_t)12 << rlog); }
+__host__ __device__ constexpr size_t slot_bytes(int rlog) { return 12 + ((size_t)8 << rlog); }
 // Shared bytes the table may take per CTA (two CTAs per SM).
 constexpr size_t kTableBudget = 96 * 1024;
 
@@ -206,6 +217,11 @@ __device__ __forceinline__ uint32_t s_addr(const void *p) { return (uint32_t)__c
 __device__ __forceinline__ uint32_t s_ld_volatile(uint32_t a) {
   uint32_t r;
   asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
+  return r;
+}
+__device__ __forceinline__ uint32_t s_add(uint32_t a, uint32_t v) {
+  uint32_t r;
+  asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(r) : "r"(a), "r"(v) : "memory");
   return r;
 }
 __device__ __forceinline__ void s_red_add(uint32_t a, uint32_t v) {
@@ -233,8 +249,8 @@ __device__ __forceinline__ uint32_t l1_home(const L1 &t, int32_t k) {
   return (((uint32_t)k * 0x9E3779B1u) >> (t.shift + 1)) << 1;
 }
 
-__device__ __forceinline__ int64_t l1_sum(uint2 ab, uint32_t c) {
-  return (int64_t)(((uint64_t)ab.y << 16) + ab.x) - (int64_t)c * (int64_t)kFlip;
+__device__ __forceinline__ int64_t l1_sum(uint64_t biased, uint32_t c) {
+  return (int64_t)biased - (int64_t)c * (int64_t)kFlip;
 }
 
 // The slow path of a row whose key is not in its home slot: probes on,
@@ -287,18 +303,17 @@ __device__ __forceinline__ void l1_row(const L1 &t, const GTable &g, int32_t k, 
   const uint32_t ea = t.ext + h * 8u;
   const uint2 e = s_ld2(ea);
   const uint32_t c = t.col(h);
-  s_red_add(t.cnt + c, 1u);
-  s_red_add(t.a + c, u & 0xffffu);
-  s_red_add(t.b + c, u >> 16);
+  const uint32_t old = s_add(t.lo + c, u);
   s_red_max_above(ea, ~u, e.x);
   s_red_max_above(ea + 4, u, e.y);
+  s_red_add(t.hi + c, 0x10000u + (old > ~u));
 }
 
 // Moves one level-1 slot to level 2.
-__device__ __forceinline__ void slot_to_l2(const GTable &g, uint4 m, uint2 ab, uint32_t *status) {
+__device__ __forceinline__ void slot_to_l2(const GTable &g, uint4 m, uint64_t biased, uint32_t *status) {
   if (m.w == 0) return;
   const int32_t k = (int32_t)(m.x ^ kFlip);
-  g_update(g, g_slot(g, k, status), m.w, l1_sum(ab, m.w), m.y, m.z);
+  g_update(g, g_slot(g, k, status), m.w, l1_sum(biased, m.w), m.y, m.z);
 }
 
 // Block-wide helpers (every thread of the CTA calls them).
@@ -309,7 +324,7 @@ __device__ __forceinline__ void l1_clear(const L1 &t, int tab, uint32_t &s_bound
 
 // level 1 -> level 2 (every occupied slot)
 __device__ __forceinline__ void l1_flush(const L1 &t, int tab, const GTable &g, uint32_t *status) {
-  for (int i = threadIdx.x; i < tab; i += kThreads) slot_to_l2(g, t.meta(i), t.sums(i), status);
+  for (int i = threadIdx.x; i < tab; i += kThreads) slot_to_l2(g, t.meta(i), t.sum(i), status);
 }
 
 // Before adding `rows` rows: if the bound on every slot's count could pass
@@ -328,7 +343,7 @@ __device__ __forceinline__ void l1_make_room(const L1 &t, int tab, const GTable 
   for (int i = threadIdx.x; i < tab; i += kThreads) {
     const uint4 m = t.meta(i);
     if (m.w > kHot) {
-      slot_to_l2(g, m, t.sums(i), status);
+      slot_to_l2(g, m, t.sum(i), status);
       t.reset(i, m.x);
       spill = true;
     } else {
@@ -479,7 +494,7 @@ __global__ void __launch_bounds__(kThreads, 2)
           const bool occ = m.w != 0;
           const unsigned b = __ballot_sync(0xffffffffu, occ);
           if (occ)
-            emit(o, pos + __popc(b & ((1u << lane) - 1)), (int32_t)(m.x ^ kFlip), m.w, l1_sum(t.sums(i), m.w),
+            emit(o, pos + __popc(b & ((1u << lane) - 1)), (int32_t)(m.x ^ kFlip), m.w, l1_sum(t.sum(i), m.w),
                  dec_min(m.y), dec_max(m.z), status);
           pos += __popc(b);
         }
@@ -588,10 +603,10 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
   GBJ_TRY(scratch.get(1, &ctr));
 
   uint32_t tslots_arg = kSlots, rlog_arg = 0;
-  // as many accumulator columns (up to 32) as the table budget allows
+  // as many accumulator columns (up to 16) as the table budget allows
   auto pick_rlog = [&]() {
     rlog_arg = 0;
-    while (rlog_arg < 5 && (size_t)tslots_arg * slot_bytes(rlog_arg + 1) <= kTableBudget) ++rlog_arg;
+    while (rlog_arg < 4 && (size_t)tslots_arg * slot_bytes(rlog_arg + 1) <= kTableBudget) ++rlog_arg;
   };
   auto launch = [&](auto kern, int tab, const int2 *pairs, uint64_t w, const uint64_t *poff,
                     const uint64_t *items, uint32_t P) -> int {

@@ -28,3 +28,13 @@ def test_partition_counts(ctx, oracle, groups):
     k[::6] = k[0]
     v = rng.integers(-1000, 1000, rows, dtype=np.int32)
     check(ctx, oracle, k, v, expected_groups=groups, strategy=2)
+
+
+@pytest.mark.parametrize("groups", [1, 16, 300, 5000])
+def test_sum_carries(ctx, oracle, groups):
+    """Sums whose low 32 bits carry at every row, at none, and once in 2^16 rows; more rows a group than a flush holds."""
+    rows = 400_001
+    k = (np.arange(rows) % groups).astype(np.int32)
+    for v in (np.full(rows, np.iinfo(np.int32).max, np.int32), np.full(rows, np.iinfo(np.int32).min, np.int32),
+              np.full(rows, -(1 << 31) + (1 << 16), np.int64).astype(np.int32)):
+        check(ctx, oracle, k, v, expected_groups=groups)
