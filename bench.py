@@ -208,6 +208,7 @@ class RadixJoin:
         return {"k_pid_hist": 4 * t,            # key read
                 "k_tile_pass": 28 * t,          # pass 1: key read + pair write (12 B),
                                                 # pass 2: pair read + pair write (16 B)
+                "k_wide_pass": 12 * t,          # 9 to 12 bits in one pass: key read + pair write
                 "k_radix_join": 8 * t}.get(name)  # partitioned pairs read once
 
     def extra(self, ms, steps, peak):
@@ -380,6 +381,7 @@ class GroupBy:
     def kernel_bytes(self, name):
         return {"k_groupby": 8 * self.n,       # (key, value) per row, raw or partitioned
                 "k_pid_hist": 4 * self.n,      # key read
+                "k_wide_pass": 16 * self.n,    # one pass: columns read + pair write
                 "k_tile_pass": 16 * self.n}.get(name)  # per pass: pair read + pair write
 
     def extra(self, ms, steps, peak):
