@@ -580,7 +580,9 @@ int nest_impl(gbj_ctx *ctx, const int64_t *d_keys, const V *d_vals, uint64_t n, 
   uint64_t slots = limit;
   if (!use_l1)
     while (slots < 4 * limit && 2 * slots * per_slot <= (32ull << 20) && (slots == limit || 16 * slots <= n)) slots *= 2;
-  GBJ_TRY(make_table(ctx, scratch, slots, d_vals != nullptr, s, &t));
+  int rc = make_table(ctx, scratch, slots, d_vals != nullptr, s, &t);
+  if (rc == GBJ_ERR_OOM && slots > limit) rc = make_table(ctx, scratch, limit, d_vals != nullptr, s, &t);
+  if (rc) return rc;
   if (use_l1) {
     // few groups: the on-chip level first (tables at 8 x groups)
     const uint32_t tslots =

@@ -814,10 +814,8 @@ int star_enqueue(gbj_star_plan *p, int slot, cudaStream_t s, bool capturing) {
 
 }  // namespace
 
-extern "C" int gbj_star_plan_create(gbj_ctx *ctx, const gbj_star_fact *fact,
-                                    const gbj_star_dim *dims, gbj_star_plan **out) {
-  if (!ctx || !out) return GBJ_ERR_INVALID;
-  *out = nullptr;
+static int make_plan(gbj_ctx *ctx, const gbj_star_fact *fact, const gbj_star_dim *dims, bool code,
+                     gbj_star_plan **out) {
   if (!fact || !dims) return set_error(ctx, GBJ_ERR_INVALID, "star: null fact or dims");
   if (fact->n_dims < 1 || fact->n_dims > kMaxDims)
     return set_error(ctx, GBJ_ERR_INVALID, "star: n_dims must be 1..4");
@@ -943,7 +941,7 @@ extern "C" int gbj_star_plan_create(gbj_ctx *ctx, const gbj_star_fact *fact,
   // the coded dimension: the largest dense one past the shared masks whose
   // classes and rows are few enough
   p->dims.coded = -1;
-  for (int d = 0; d < fact->n_dims; ++d) {
+  for (int d = 0; d < fact->n_dims && code; ++d) {
     const DimDev &dd = p->dims.d[d];
     const gbj_star_dim &hd = dims[d];
     if (dd.smem_off >= 0 || dd.kind || dd.n > kCodedRows || dd.n_attrs < 1) continue;
@@ -1077,6 +1075,15 @@ extern "C" int gbj_star_plan_create(gbj_ctx *ctx, const gbj_star_fact *fact,
   if (e != cudaSuccess) return fail(cuda_error(ctx, e, "cudaStreamSynchronize"));
   *out = p;
   return GBJ_OK;
+}
+
+extern "C" int gbj_star_plan_create(gbj_ctx *ctx, const gbj_star_fact *fact,
+                                    const gbj_star_dim *dims, gbj_star_plan **out) {
+  if (!ctx || !out) return GBJ_ERR_INVALID;
+  *out = nullptr;
+  const int rc = make_plan(ctx, fact, dims, true, out);
+  // a pool without room for the codes: a plan without them
+  return rc == GBJ_ERR_OOM ? make_plan(ctx, fact, dims, false, out) : rc;
 }
 
 extern "C" int gbj_star_run(gbj_star_plan *p, const gbj_star_query *queries, int32_t n_queries,

@@ -63,3 +63,23 @@ def test_long_chains(ctx, oracle):
     order = np.argsort(host(got[0])[:m])
     for g, e in zip(got[:5], oracle.nest_i64(keys, vals)):
         assert (host(g)[:m][order] == e).all()
+
+
+def test_table_at_the_pool_limit(ctx, oracle):
+    """Where the pool has no room for a table of four times the slots, one of the least size is taken."""
+    rng = np.random.default_rng(3)
+    keys = rng.integers(0, 1 << 40, 4096)[rng.integers(0, 4096, 1 << 19)]
+    vals = rng.integers(-1000, 1000, 1 << 19)
+    dk, dv = dev(keys), dev(vals)
+    ctx.sync()
+    # 8192 slots (two for each group) of 48 bytes and the one of INT64_MIN; 32,768 would be 1.5 MB
+    ctx.set_pool_limit(ctx.pool_stats()["in_use"] + 48 * 8193 + (1 << 16))
+    try:
+        got = ctx.nest_i64(dk, dv, 5000, expected_groups=4096)
+        ctx.sync()
+    finally:
+        ctx.set_pool_limit(0)
+    m = int(host(got[5])[0])
+    order = np.argsort(host(got[0])[:m])
+    for g, e in zip(got[:5], oracle.nest_i64(keys, vals)):
+        assert (host(g)[:m][order] == e).all()

@@ -63,3 +63,31 @@ def test_coded(ctx, oracle, n_fact, shift, stray, spans, rows, use_graph):
                 exp = oracle.star_query(data, q)
                 assert len(got[0]) == len(exp[0]) and all((x == y).all() for x, y in zip(got, exp))
     plan.close()
+
+
+def test_without_room_for_the_codes(ctx, oracle):
+    """A plan that the pool has room for without the codes is made without them."""
+    rng = np.random.default_rng(8)
+    dims = [dim("big", 70_000, (20, 7), rng), dim("coded", 65_536, (25, 5), rng)]
+    fk = [rng.integers(0, d.n, 50_001).astype(np.int32) for d in dims]
+    qty, price = rng.integers(1, 51, 50_001).astype(np.int32), rng.integers(-1000, 1000, 50_001).astype(np.int32)
+    data = star.StarData(dims, fk, qty, price)
+    cols = ([torch.from_numpy(c).cuda() for c in fk], torch.from_numpy(qty).cuda(), torch.from_numpy(price).cuda())
+    ctx.sync()
+    before = ctx.pool_stats()["in_use"]
+    plan = star.StarPlan(ctx, data, fact_tensors=cols)
+    ctx.sync()
+    need = ctx.pool_stats()["in_use"] - before
+    plan.close()
+    ctx.sync()
+    ctx.set_pool_limit(ctx.pool_stats()["in_use"] + need - 40_000)
+    try:
+        plan = star.StarPlan(ctx, data, fact_tensors=cols)
+        assert ctx.pool_stats()["in_use"] - before <= need - 40_000
+    finally:
+        ctx.set_pool_limit(0)
+    q = query(dims, (0, 1), {1: (0, 0, 12)}, ((1, 0), (0, 1)))
+    got = star.StarPlan.results(plan.run([q]), 1)[0]
+    exp = oracle.star_query(data, q)
+    assert len(got[0]) == len(exp[0]) and all((x == y).all() for x, y in zip(got, exp))
+    plan.close()
