@@ -39,3 +39,20 @@ def test_lists(ctx, oracle, dtype, unique, n_probe, n_aggs):
     t.destroy()
     join = oracle.join_agg_i64 if dtype == np.int64 else oracle.join_agg
     assert got == join(rk, rp, sk, sp, aggs)
+
+
+@pytest.mark.parametrize("n_build,copies", [(16, 1), (16, 16), (4000, 1), (8192, 1), (8192, 2), (8191, 5)])
+def test_marked_buckets(ctx, oracle, n_build, copies):
+    """int64 tables at load one half: rows that go past one and several full buckets are found, with the build rows
+    of both slots of a marked bucket."""
+    rng = np.random.default_rng(n_build + copies)
+    rk = rng.permutation(np.arange(n_build) // copies).astype(np.int64) * 0x1_0000_0003
+    rp = rng.integers(-1000, 1000, n_build).astype(np.int32)
+    sk = rng.permutation(np.concatenate([rk[:3000], rk[:3000] + 1, rk[-3000:]]))
+    sp = rng.integers(-1000, 1000, len(sk)).astype(np.int32)
+    aggs = [(abi.AGG_COUNT, abi.VAL_ONE), (abi.AGG_SUM, abi.VAL_PRODUCT), (abi.AGG_SUM, abi.VAL_ROWID_XOR)]
+    t = ctx.join_build(dev(rk), dev(rp))
+    got = host(ctx.join_probe_agg(t, dev(sk), dev(sp), aggs)).tolist()
+    ctx.sync()
+    t.destroy()
+    assert got == oracle.join_agg_i64(rk, rp, sk, sp, aggs)
