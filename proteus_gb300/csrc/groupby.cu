@@ -8,10 +8,10 @@
 //
 // GB300 design:
 //  * level 1 is one open-addressing table of up to 4096 slots per CTA in
-//    shared memory, updated with 32-bit atomics only (count, and the sum as
-//    two 16-bit halves of the biased value, which stay exact while a slot
-//    takes at most 65535 rows between flushes; hot slots move to level 2
-//    before that).  Min and max atomics are issued only when the value
+//    shared memory, updated with 32-bit atomics only (the sum's low word, and
+//    a word of its carries and the rows, exact while a slot takes at most
+//    65535 rows between flushes; hot slots move to level 2 before that).
+//    Min and max atomics are issued only when the value
 //    improves the stored extreme, so they fade out as a group fills;
 //  * level 2 is a global open-addressing table that receives level 1 when a
 //    CTA finishes (and rows that find level 1 full), with integer atomics,

@@ -5,7 +5,7 @@
 // GpuHashJoinChained (core/olap/lib/operators/hash-join-chained.cpp:262-566,
 // core/olap/lib/operators/gpu/gpu-hash-join-chained.cpp:31-73).  The
 // reference chains entries behind a head array; here the table is an array
-// of 32-byte buckets of four slots (keys, then payloads or rows + 1) sized
+// of 32-byte buckets of four slots {key, payload or row + 1} sized
 // to a power of two with load factor <= 1/2, so a probe is one L2 sector in
 // the common case and the table for a 2^20-row build side (16 MiB) stays
 // resident in the 129 MB L2 while the probe side streams from HBM.  The

@@ -14,8 +14,8 @@
 //    Each kernel is a persistent grid that takes items from one atomic
 //    counter; an item is a fixed-size chunk of one query's rows or slots,
 //    so big and small queries share the SMs without per-query launches;
-//  * the join table is open addressing with one 64-bit slot per build row
-//    holding {key | group slot << 32} (load factor <= 0.5), and duplicate
+//  * the join table is open addressing in sectors of four 64-bit slots, one
+//    slot per build row {key | group slot << 32} (load factor <= 0.5); duplicate
 //    build keys keep HashJoinChained's every-match semantics.  A slot whose
 //    key half is INT32_MIN is empty; build rows with that key go to a side
 //    list that probes of INT32_MIN walk;
