@@ -651,7 +651,7 @@ __device__ __forceinline__ JBucket64 ld_bucket64(const JBucket64 *p) {
 // from marked buckets only, where a full bucket used to send every probe of a
 // key that is not unique to the next one (1.5 M rows, two a key, 20 M probes:
 // 541 -> 391 us; unique keys, half of the probes without a match: 224 -> 208;
-// the build takes 74 -> 77 and 50 -> 51).
+// the build, with its clear, takes 85 and 51 us, 74 and 50 without the marks).
 __global__ void __launch_bounds__(kThreads)
     k_jb64_build(const int64_t *__restrict__ keys, const int32_t *__restrict__ payload, uint64_t n,
                  JBucket64 *__restrict__ bk, uint64_t bmask, uint32_t *__restrict__ meta,
@@ -686,7 +686,8 @@ __global__ void __launch_bounds__(kThreads)
           dup |= old == kf;
         }
       }
-      if (!placed) atomicOr(&bk[b].x[1].y, INT32_MIN);
+      // 64 bits wide, as the row's own word that may be written meanwhile
+      if (!placed) atomicOr(reinterpret_cast<unsigned long long *>(&bk[b].x[1]), 1ull << 63);
       b = (b + 1) & bmask;
     }
     if (!placed) gbjd::latch(status, GBJ_DEV_CAPACITY);
