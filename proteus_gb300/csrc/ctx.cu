@@ -3,7 +3,7 @@
 // The pool replaces the reference's MemoryManager slab allocators and the
 // buffer-manager's 2 MiB block pools (core/platform/lib/memory/
 // memory-manager.cpp, buffer-manager.cu): one cudaMalloc at context creation,
-// then host-side best-fit bookkeeping.  Scratch of every entry point comes
+// then host-side best-fit bookkeeping (pool.h).  Scratch of every entry point comes
 // from it, so steady-state calls never allocate device memory.
 #include <cstdio>
 #include <cstring>
@@ -78,59 +78,6 @@ static void prof_collect(gbj_ctx *ctx) {
 
 static constexpr uint64_t kAlign = 256;
 
-static void pool_insert_free(Pool &p, uint64_t off, uint64_t size) {
-  auto it = p.free_by_off.lower_bound(off);
-  if (it != p.free_by_off.end() && off + size == it->first) {
-    size += it->second;
-    it = p.free_by_off.erase(it);
-  }
-  if (it != p.free_by_off.begin()) {
-    auto prev = std::prev(it);
-    if (prev->first + prev->second == off) {
-      prev->second += size;
-      return;
-    }
-  }
-  p.free_by_off.emplace(off, size);
-}
-
-// Moves deferred blocks whose work is done (or that belong to `s`) back to
-// the free map.  `wait` blocks on pending events of other streams.
-static void pool_reclaim(Pool &p, cudaStream_t s, bool wait) {
-  std::vector<Pool::Deferred> keep;
-  for (auto &d : p.deferred) {
-    bool ok = (d.stream == s);
-    if (!ok) {
-      cudaError_t q = wait ? cudaEventSynchronize(d.ev) : cudaEventQuery(d.ev);
-      ok = (q == cudaSuccess);
-      if (q != cudaSuccess && q != cudaErrorNotReady) (void)cudaGetLastError();
-    }
-    if (ok) {
-      // Same-stream reuse is ordered after the recorded point; the event
-      // is no longer needed either way.
-      cudaEventDestroy(d.ev);
-      pool_insert_free(p, d.off, d.size);
-    } else {
-      keep.push_back(d);
-    }
-  }
-  p.deferred.swap(keep);
-}
-
-static bool pool_take(Pool &p, uint64_t size, uint64_t *off) {
-  auto best = p.free_by_off.end();
-  for (auto it = p.free_by_off.begin(); it != p.free_by_off.end(); ++it)
-    if (it->second >= size && (best == p.free_by_off.end() || it->second < best->second))
-      best = it;
-  if (best == p.free_by_off.end()) return false;
-  *off = best->first;
-  uint64_t rest = best->second - size;
-  uint64_t roff = best->first + size;
-  p.free_by_off.erase(best);
-  if (rest) p.free_by_off.emplace(roff, rest);
-  return true;
-}
-
 int pool_alloc(gbj_ctx *ctx, uint64_t bytes, cudaStream_t s, void **out) {
   if (!out) return set_error(ctx, GBJ_ERR_INVALID, "pool_alloc: null out");
   std::lock_guard<std::mutex> g(ctx->mu);
@@ -142,15 +89,11 @@ int pool_alloc(gbj_ctx *ctx, uint64_t bytes, cudaStream_t s, void **out) {
     return set_error(ctx, GBJ_ERR_OOM,
                      "device pool limit reached: requested " + std::to_string(bytes) + " B, in use " +
                          std::to_string(p.in_use) + " of the " + std::to_string(p.limit) + " B limit");
-  pool_reclaim(p, s, false);
-  if (!pool_take(p, size, &off)) {
-    pool_reclaim(p, s, true);
-    if (!pool_take(p, size, &off))
-      return set_error(ctx, GBJ_ERR_OOM,
-                       "device pool exhausted: requested " + std::to_string(bytes) +
-                           " B, in use " + std::to_string(p.in_use) + " of " +
-                           std::to_string(p.capacity) + " B");
-  }
+  if (!pool_take(p, size, s, &off))
+    return set_error(ctx, GBJ_ERR_OOM,
+                     "device pool exhausted: requested " + std::to_string(bytes) +
+                         " B, in use " + std::to_string(p.in_use) + " of " +
+                         std::to_string(p.capacity) + " B");
   p.used[off] = size;
   p.in_use += size;
   if (p.in_use > p.peak) p.peak = p.in_use;
@@ -169,17 +112,7 @@ int pool_release(gbj_ctx *ctx, void *ptr, cudaStream_t s) {
   uint64_t size = it->second;
   p.used.erase(it);
   p.in_use -= size;
-  cudaEvent_t ev;
-  if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventRecord(ev, s) != cudaSuccess) {
-    // Capturing streams cannot be queried: fall back to a full sync.
-    (void)cudaGetLastError();
-    cudaStreamSynchronize(s);
-    (void)cudaGetLastError();
-    pool_insert_free(p, off, size);
-    return GBJ_OK;
-  }
-  p.deferred.push_back({off, size, s, ev});
+  pool_give(p, off, size, s);
   return GBJ_OK;
 }
 
@@ -279,7 +212,7 @@ int gbj_ctx_destroy(gbj_ctx *ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   prof_collect(ctx);
-  for (auto &d : ctx->pool.deferred) cudaEventDestroy(d.ev);
+  for (auto &d : ctx->pool.deferred) cudaEventDestroy(d.second.ev);
   cudaFree(ctx->pool.base);
   cudaStreamDestroy(ctx->stream);
   delete ctx;

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "gbjoin.h"
+#include "pool.h"
 
 // ----------------------------------------------------------------- status
 // Device-side error bits latched into the context's status word; gbj_sync
@@ -25,25 +26,6 @@ enum : uint32_t {
 
 // Upper bound on the iterations of any device-side spin (bounded waits).
 constexpr uint32_t kSpinLimit = 1u << 22;
-
-struct Pool {
-  // Best-fit allocator over one cudaMalloc'd block.  Freed blocks stay
-  // "deferred" behind a CUDA event until the stream that used them has
-  // passed that point; a request on the same stream may reuse them at once
-  // (stream order), a request on another stream reclaims them once the
-  // event has completed (or waits on it when nothing else fits).
-  char *base = nullptr;
-  uint64_t capacity = 0, in_use = 0, peak = 0;
-  uint64_t limit = 0;  // gbj_ctx_set_pool_limit: most bytes handed out (0 = capacity)
-  std::map<uint64_t, uint64_t> free_by_off;  // offset -> size
-  std::unordered_map<uint64_t, uint64_t> used;  // offset -> size
-  struct Deferred {
-    uint64_t off, size;
-    cudaStream_t stream;
-    cudaEvent_t ev;
-  };
-  std::vector<Deferred> deferred;
-};
 
 struct gbj_ctx {
   int device = 0;
