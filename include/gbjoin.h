@@ -183,6 +183,9 @@ int gbj_join_probe_pairs_i64(gbj_ctx *ctx, const gbj_table *table,
                              int32_t *d_out_probe_rows, uint64_t capacity,
                              uint64_t *d_count, void *stream);
 
+/* Needs no synchronisation: the table's memory is used again behind the builds
+ * and probes that were enqueued, on whatever streams (a graph that captured a
+ * probe needs the table for as long as it is replayed). */
 int gbj_table_destroy(gbj_ctx *ctx, gbj_table *table);
 /* Number of slots of the table (host query). */
 uint64_t gbj_table_slots(const gbj_table *table);

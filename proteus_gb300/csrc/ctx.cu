@@ -101,18 +101,38 @@ int pool_alloc(gbj_ctx *ctx, uint64_t bytes, cudaStream_t s, void **out) {
   return GBJ_OK;
 }
 
+// Ends the use of a block in the books; *off, *size: its range.
+static int pool_end(gbj_ctx *ctx, void *ptr, uint64_t *off, uint64_t *size) {
+  Pool &p = ctx->pool;
+  *off = (uint64_t)((char *)ptr - p.base);
+  auto it = p.used.find(*off);
+  if ((char *)ptr < p.base || it == p.used.end())
+    return set_error(ctx, GBJ_ERR_INVALID, "pool_free: pointer not from this pool");
+  *size = it->second;
+  p.used.erase(it);
+  p.in_use -= *size;
+  return GBJ_OK;
+}
+
 int pool_release(gbj_ctx *ctx, void *ptr, cudaStream_t s) {
   if (!ptr) return GBJ_OK;
   std::lock_guard<std::mutex> g(ctx->mu);
-  Pool &p = ctx->pool;
-  uint64_t off = (uint64_t)((char *)ptr - p.base);
-  auto it = p.used.find(off);
-  if ((char *)ptr < p.base || it == p.used.end())
-    return set_error(ctx, GBJ_ERR_INVALID, "pool_free: pointer not from this pool");
-  uint64_t size = it->second;
-  p.used.erase(it);
-  p.in_use -= size;
-  pool_give(p, off, size, s);
+  uint64_t off, size;
+  GBJ_TRY(pool_end(ctx, ptr, &off, &size));
+  pool_give(ctx->pool, off, size, s);
+  return GBJ_OK;
+}
+
+void note_use(gbj_ctx *ctx, BlockUses &uses, cudaStream_t s) {
+  std::lock_guard<std::mutex> g(ctx->mu);
+  pool_note_use(uses, s);
+}
+
+int pool_release_used(gbj_ctx *ctx, void *ptr, BlockUses &uses) {
+  std::lock_guard<std::mutex> g(ctx->mu);
+  uint64_t off, size;
+  GBJ_TRY(pool_end(ctx, ptr, &off, &size));
+  pool_give(ctx->pool, off, size, std::move(uses));
   return GBJ_OK;
 }
 
@@ -212,7 +232,8 @@ int gbj_ctx_destroy(gbj_ctx *ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   prof_collect(ctx);
-  for (auto &d : ctx->pool.deferred) cudaEventDestroy(d.second.ev);
+  for (auto &d : ctx->pool.deferred)
+    for (auto &u : d.second.uses) cudaEventDestroy(u.second);
   cudaFree(ctx->pool.base);
   cudaStreamDestroy(ctx->stream);
   delete ctx;

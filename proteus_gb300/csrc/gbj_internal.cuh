@@ -66,6 +66,7 @@ struct gbj_table {
   const int32_t *payload = nullptr;
   uint64_t n = 0;
   bool i64 = false;  // int64 keys (gbj_join_build_i64): 2-slot buckets
+  mutable BlockUses uses;  // the build and the probes
 };
 
 // ------------------------------------------------------------ host helpers
@@ -77,6 +78,10 @@ cudaStream_t pick_stream(gbj_ctx *ctx, void *stream);
 int pool_alloc(gbj_ctx *ctx, uint64_t bytes, cudaStream_t s, void **out);
 // Releases after the work already enqueued on `s` (records an event).
 int pool_release(gbj_ctx *ctx, void *p, cudaStream_t s);
+// For a block that outlives a call and is used on any stream: note_use after
+// each launch that uses it, then a release behind all of those.
+void note_use(gbj_ctx *ctx, BlockUses &uses, cudaStream_t s);
+int pool_release_used(gbj_ctx *ctx, void *p, BlockUses &uses);
 
 // Scratch allocations owned by one entry-point call; released (deferred on
 // the call's stream) when the scope ends.

@@ -1268,13 +1268,14 @@ int gbj_join_build(gbj_ctx *ctx, const int32_t *d_keys,
       if (rc) return fail(rc);
     }
   }
+  note_use(ctx, t->uses, s);
   *out = t;
   return GBJ_OK;
 }
 
 int gbj_table_destroy(gbj_ctx *ctx, gbj_table *table) {
   if (!ctx || !table) return GBJ_ERR_INVALID;
-  int rc = pool_release(ctx, table->slots, ctx->stream);
+  const int rc = pool_release_used(ctx, table->slots, table->uses);
   delete table;
   return rc;
 }
@@ -1301,7 +1302,9 @@ int gbj_join_probe_agg(gbj_ctx *ctx, const gbj_table *t, const int32_t *d_keys,
   GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
   if (n == 0) return GBJ_OK;
   launch_jb_probe(ctx->sm_count, t, d_keys, d_payload, n, spec, d_out, s);
-  return after_launch(ctx, "k_jb_probe_agg", s);
+  const int rc = after_launch(ctx, "k_jb_probe_agg", s);
+  note_use(ctx, t->uses, s);
+  return rc;
 }
 
 int gbj_join_probe_pairs(gbj_ctx *ctx, const gbj_table *t, const int32_t *d_keys,
@@ -1320,7 +1323,9 @@ int gbj_join_probe_pairs(gbj_ctx *ctx, const gbj_table *t, const int32_t *d_keys
   const uint64_t nbk = (t->mask + 1) / 4;
   if (t->rows) launch_jb_pairs<JLayout32<true>>(ctx->sm_count, t, nbk, d_keys, d_probe_rows, n, po, s);
   else launch_jb_pairs<JLayout32<false>>(ctx->sm_count, t, nbk, d_keys, d_probe_rows, n, po, s);
-  return after_launch(ctx, "k_jb_probe_pairs", s);
+  const int rc = after_launch(ctx, "k_jb_probe_pairs", s);
+  note_use(ctx, t->uses, s);
+  return rc;
 }
 
 int gbj_join_build_i64(gbj_ctx *ctx, const int64_t *d_keys, const int32_t *d_payload, uint64_t n,
@@ -1372,6 +1377,7 @@ int gbj_join_build_i64(gbj_ctx *ctx, const int64_t *d_keys, const int32_t *d_pay
       return rc;
     }
   }
+  note_use(ctx, t->uses, s);
   *out = t;
   return GBJ_OK;
 }
@@ -1395,7 +1401,9 @@ int gbj_join_probe_agg_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_ke
   GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
   if (n == 0) return GBJ_OK;
   launch_jb_list<JLayout64>(ctx->sm_count, t, (t->mask + 1) / 2, d_keys, d_payload, n, spec, d_out, s);
-  return after_launch(ctx, "k_jb_probe_list", s);
+  const int rc = after_launch(ctx, "k_jb_probe_list", s);
+  note_use(ctx, t->uses, s);
+  return rc;
 }
 
 int gbj_join_probe_pairs_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_keys,
@@ -1410,7 +1418,9 @@ int gbj_join_probe_pairs_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_
   if (n == 0) return GBJ_OK;
   const PairOut po{d_build_rows, d_out_probe_rows, capacity, (unsigned long long *)d_count, ctx->d_status};
   launch_jb_pairs<JLayout64>(ctx->sm_count, t, (t->mask + 1) / 2, d_keys, d_probe_rows, n, po, s);
-  return after_launch(ctx, "k_jb_probe_pairs", s);
+  const int rc = after_launch(ctx, "k_jb_probe_pairs", s);
+  note_use(ctx, t->uses, s);
+  return rc;
 }
 
 int gbj_reduce(gbj_ctx *ctx, const int32_t *d_col, const int32_t *d_rows,

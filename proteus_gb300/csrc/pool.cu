@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <iterator>
+#include <utility>
 
 namespace gbj {
 namespace {
@@ -23,10 +24,32 @@ void insert_free(Pool &p, uint64_t off, uint64_t size) {
   p.free_by_off.emplace(off, size);
 }
 
-bool completed(const Pool::Deferred &d, bool wait) {
-  const cudaError_t q = wait ? cudaEventSynchronize(d.ev) : cudaEventQuery(d.ev);
+bool completed(cudaEvent_t ev, bool wait) {
+  const cudaError_t q = wait ? cudaEventSynchronize(ev) : cudaEventQuery(ev);
   if (q != cudaSuccess && q != cudaErrorNotReady) (void)cudaGetLastError();
   return q == cudaSuccess;
+}
+
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// Drops the uses that have ended; true: all of them.
+bool ended(BlockUses &uses, bool wait) {
+  for (auto it = uses.begin(); it != uses.end();) {
+    if (completed(it->second, wait)) {
+      cudaEventDestroy(it->second);
+      it = uses.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  return uses.empty();
+}
+void drop(BlockUses &uses) {
+  for (auto &u : uses) cudaEventDestroy(u.second);
 }
 
 // Frees the other streams' ranges whose work is done; `wait` waits for it.  A
@@ -34,9 +57,9 @@ bool completed(const Pool::Deferred &d, bool wait) {
 // request on its stream.
 void reclaim(Pool &p, cudaStream_t s, bool wait) {
   for (auto it = p.deferred.begin(); it != p.deferred.end();) {
-    const Pool::Deferred &d = it->second;
-    if (d.stream == s ? d.captured : completed(d, wait)) {
-      cudaEventDestroy(d.ev);
+    Pool::Deferred &d = it->second;
+    if (d.of(s) ? d.captured : ended(d.uses, wait)) {
+      drop(d.uses);
       insert_free(p, it->first, d.size);
       it = p.deferred.erase(it);
     } else {
@@ -57,7 +80,7 @@ bool fit(const Pool &p, uint64_t size, cudaStream_t s, uint64_t *off) {
     }
   };
   for (;;) {
-    while (d != p.deferred.end() && d->second.stream != s) ++d;
+    while (d != p.deferred.end() && !d->second.of(s)) ++d;
     const bool has_f = f != p.free_by_off.end(), has_d = d != p.deferred.end();
     if (!has_f && !has_d) break;
     uint64_t o, n;
@@ -87,14 +110,14 @@ void carve(Pool &p, uint64_t off, uint64_t size, cudaStream_t s) {
     if (e > end) p.free_by_off.emplace(end, e - end);
   }
   for (auto it = p.deferred.lower_bound(off); it != p.deferred.end() && it->first < end;) {
-    Pool::Deferred d = it->second;
+    Pool::Deferred d = std::move(it->second);
     const uint64_t e = it->first + d.size;
     it = p.deferred.erase(it);
     if (e > end) {
       d.size = e - end;
-      p.deferred.emplace(end, d);
+      p.deferred.emplace(end, std::move(d));
     } else {
-      cudaEventDestroy(d.ev);
+      drop(d.uses);
     }
   }
 }
@@ -111,43 +134,69 @@ bool pool_take(Pool &p, uint64_t size, cudaStream_t s, uint64_t *off) {
   return true;
 }
 
-void pool_give(Pool &p, uint64_t off, uint64_t size, cudaStream_t s) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) (void)cudaGetLastError();
-  Pool::Deferred d{size, s, nullptr, cap != cudaStreamCaptureStatusNone};
-  if (cudaEventCreateWithFlags(&d.ev, cudaEventDisableTiming) != cudaSuccess || cudaEventRecord(d.ev, s) != cudaSuccess) {
-    // an event that cannot be recorded: fall back to a full sync
-    (void)cudaGetLastError();
-    if (d.ev) cudaEventDestroy(d.ev);
-    cudaStreamSynchronize(s);
-    (void)cudaGetLastError();
-    insert_free(p, off, size);
-    return;
-  }
-  // ranges of s beside it: free when their work is done, else one range with
-  // it, behind the later event
-  auto merges = [&](const Pool::Deferred &o) { return o.stream == s && !o.captured && !d.captured; };
+static void defer(Pool &p, uint64_t off, Pool::Deferred d) {
+  // ranges of the same stream beside it: free when their work is done, else
+  // one range with it, behind the later event
+  auto merges = [&](const Pool::Deferred &o) {
+    return d.uses.size() == 1 && o.of(d.uses[0].first) && !o.captured && !d.captured;
+  };
   auto it = p.deferred.lower_bound(off);
-  if (it != p.deferred.end() && it->first == off + size && merges(it->second)) {
-    if (completed(it->second, false)) insert_free(p, it->first, it->second.size);
+  if (it != p.deferred.end() && it->first == off + d.size && merges(it->second)) {
+    if (completed(it->second.uses[0].second, false)) insert_free(p, it->first, it->second.size);
     else d.size += it->second.size;
-    cudaEventDestroy(it->second.ev);
+    drop(it->second.uses);
     it = p.deferred.erase(it);
   }
   if (it != p.deferred.begin()) {
     auto prev = std::prev(it);
     if (prev->first + prev->second.size == off && merges(prev->second)) {
-      if (completed(prev->second, false)) {
+      if (completed(prev->second.uses[0].second, false)) {
         insert_free(p, prev->first, prev->second.size);
       } else {
         off = prev->first;
         d.size += prev->second.size;
       }
-      cudaEventDestroy(prev->second.ev);
+      drop(prev->second.uses);
       p.deferred.erase(prev);
     }
   }
-  p.deferred.emplace(off, d);
+  p.deferred.emplace(off, std::move(d));
+}
+
+void pool_give(Pool &p, uint64_t off, uint64_t size, cudaStream_t s) {
+  const bool cap = capturing(s);
+  cudaEvent_t ev = nullptr;
+  if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess || cudaEventRecord(ev, s) != cudaSuccess) {
+    // an event that cannot be recorded: fall back to a full sync
+    (void)cudaGetLastError();
+    if (ev) cudaEventDestroy(ev);
+    cudaStreamSynchronize(s);
+    (void)cudaGetLastError();
+    insert_free(p, off, size);
+    return;
+  }
+  defer(p, off, {size, {{s, ev}}, cap});
+}
+
+void pool_give(Pool &p, uint64_t off, uint64_t size, BlockUses uses) {
+  if (ended(uses, false)) insert_free(p, off, size);
+  else defer(p, off, {size, std::move(uses), false});
+}
+
+void pool_note_use(BlockUses &uses, cudaStream_t s) {
+  if (capturing(s)) return;
+  cudaEvent_t ev = nullptr;
+  for (auto &u : uses)
+    if (u.first == s) ev = u.second;
+  if (!ev) {
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) uses.push_back({s, ev});
+    else ev = nullptr;
+  }
+  if (!ev || cudaEventRecord(ev, s) != cudaSuccess) {  // nothing left in flight instead
+    (void)cudaGetLastError();
+    cudaStreamSynchronize(s);
+    (void)cudaGetLastError();
+  }
 }
 
 }  // namespace gbj

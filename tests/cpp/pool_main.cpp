@@ -3,7 +3,9 @@
 // A range handed out must not be in use by unfinished work of another stream.
 #include <cstdio>
 #include <cstdlib>
+#include <initializer_list>
 #include <random>
+#include <utility>
 #include <vector>
 
 #include "pool.h"
@@ -95,13 +97,22 @@ struct Model {
     held.erase(held.begin() + (long)i);
     gbj::pool_give(p, b.off, b.size, stream(s));
   }
+  // given back behind all that streams a, b, .. were last made to do with it
+  void give_used(size_t i, std::initializer_list<int> streams) {
+    BlockUses uses;
+    for (int s : streams) use(i, s), gbj::pool_note_use(uses, stream(s));
+    const Block b = held[i];
+    held.erase(held.begin() + (long)i);
+    gbj::pool_give(p, b.off, b.size, std::move(uses));
+  }
   // every byte is in exactly one place
   void check() {
     uint64_t sum = 0;
     for (auto &f : p.free_by_off) sum += f.second;
-    for (auto &d : p.deferred) sum += d.second.size;
+    int events = 0;
+    for (auto &d : p.deferred) sum += d.second.size, events += (int)d.second.uses.size();
     for (const Block &b : held) sum += b.size;
-    if (sum != kUnit * kUnits || live_events != (int)p.deferred.size()) {
+    if (sum != kUnit * kUnits || live_events != events) {
       printf("bytes or events lost\n");
       exit(1);
     }
@@ -134,6 +145,16 @@ int main() {
     require(m.take(kUnits, 0) && waits == w, "adjacent ranges were not used together");
     m.check();
   }
+  {  // a block that two streams use: the one whose work has ended does not free it
+    Model m;
+    m.take(kUnits, 0), m.use(0, 0);
+    m.give_used(0, {0, 1, 0});
+    done[1] = issued[1];
+    const int w = waits;
+    require(m.take(4, 0) && waits == w, "the one stream left waited");
+    require(m.take(4, 2) && waits == w + 1, "a third stream did not wait");
+    m.check();
+  }
   for (unsigned seed = 0; seed < 300; ++seed) {
     Model m;
     std::mt19937 rng(seed);
@@ -145,13 +166,13 @@ int main() {
           if (m.take(1 + rng() % (seed % 2 ? 40 : 8), s)) m.use(m.held.size() - 1, s), m.give(m.held.size() - 1, s);
           break;
         case 2:
-          if (m.held.size() < 6 && m.take(1 + rng() % 8, s)) m.use(m.held.size() - 1, s);
+          if (m.held.size() < 6) m.take(1 + rng() % 8, s);
           break;
-        case 3:  // a block kept for a while, given back on the stream that waited for all its users
+        case 3:  // a block that several streams have used for a while
           if (!m.held.empty()) {
             const size_t i = rng() % m.held.size();
-            for (int o = 0; o < 3; ++o) cudaStreamSynchronize(stream(o));
-            m.use(i, s), m.give(i, s);
+            const int o = (int)(rng() % 3);
+            m.give_used(i, {0, 1, 2, s, o, s});
           }
           break;
         case 4:
@@ -164,7 +185,8 @@ int main() {
     while (!m.held.empty()) m.give(0, 0);
     require(m.take(kUnits, 3), "not everything came back");
     m.give(0, 3);
-    for (auto &d : m.p.deferred) cudaEventDestroy(d.second.ev);
+    for (auto &d : m.p.deferred)
+      for (auto &u : d.second.uses) cudaEventDestroy(u.second);
     m.p.deferred.clear();
   }
   printf("ok\n");
