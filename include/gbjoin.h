@@ -341,6 +341,7 @@ int gbj_bloom_build(gbj_ctx *ctx, const int32_t *d_keys, uint64_t n,
 int gbj_bloom_probe(gbj_ctx *ctx, const gbj_bloom *filter,
                     const int32_t *d_keys, uint64_t n, int32_t *d_rows_out,
                     uint64_t *d_count, void *stream);
+/* As gbj_table_destroy: behind the build and the probes, on any stream. */
 int gbj_bloom_destroy(gbj_ctx *ctx, gbj_bloom *filter);
 
 /* ---------------------------------------------------------- hash rearrange */

@@ -21,6 +21,7 @@ using namespace gbj;
 struct gbj_bloom {
   uint32_t *bits = nullptr;  // pool block
   uint64_t size = 0;         // positions (power of two)
+  mutable BlockUses uses;    // the build and the probes
 };
 
 namespace {
@@ -62,7 +63,12 @@ extern "C" int gbj_bloom_build(gbj_ctx *ctx, const int32_t *d_keys, uint64_t n, 
     delete f;
     return rc;
   }
-  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(f->bits, 0, filter_size / 8, s));
+  const cudaError_t e = cudaMemsetAsync(f->bits, 0, filter_size / 8, s);
+  if (e != cudaSuccess) {
+    pool_release(ctx, f->bits, s);
+    delete f;
+    return cuda_error(ctx, e, "cudaMemsetAsync(bloom)");
+  }
   if (n) {
     const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx->sm_count * 16);
     k_bloom_build<<<grid, 256, 0, s>>>(d_keys, n, (uint32_t)(filter_size - 1), f->bits);
@@ -73,6 +79,7 @@ extern "C" int gbj_bloom_build(gbj_ctx *ctx, const int32_t *d_keys, uint64_t n, 
       return r;
     }
   }
+  note_use(ctx, f->uses, s);
   *out = f;
   return GBJ_OK;
 }
@@ -83,13 +90,15 @@ extern "C" int gbj_bloom_probe(gbj_ctx *ctx, const gbj_bloom *filter, const int3
   if (n >= (1ull << 31)) return set_error(ctx, GBJ_ERR_INVALID, "bloom: n >= 2^31");
   cudaStream_t s = pick_stream(ctx, stream);
   prof_mark(ctx, s);
-  return compact_rows(ctx, BloomPred{d_keys, filter->bits, (uint32_t)(filter->size - 1)}, n, d_rows_out,
-                      d_count, s);
+  const int rc = compact_rows(ctx, BloomPred{d_keys, filter->bits, (uint32_t)(filter->size - 1)}, n, d_rows_out,
+                              d_count, s);
+  note_use(ctx, filter->uses, s);
+  return rc;
 }
 
 extern "C" int gbj_bloom_destroy(gbj_ctx *ctx, gbj_bloom *filter) {
   if (!ctx || !filter) return GBJ_ERR_INVALID;
-  pool_release(ctx, filter->bits, ctx->stream);
+  const int rc = pool_release_used(ctx, filter->bits, filter->uses);
   delete filter;
-  return GBJ_OK;
+  return rc;
 }
