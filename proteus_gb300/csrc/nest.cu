@@ -594,7 +594,8 @@ int nest_impl(gbj_ctx *ctx, const int64_t *d_keys, const V *d_vals, uint64_t n, 
     GBJ_TRY(scratch.get(1, &ctr));
     GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
     auto kern = k_nest_l1<V>;
-    GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most any call takes: the limit is the kernel's, not the call's
+    GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kL1Budget));
     int per_sm = 1;
     GBJ_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kL1Threads, smem));
     per_sm = std::max(per_sm, 1);

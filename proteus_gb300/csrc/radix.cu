@@ -1085,8 +1085,9 @@ int partition_impl(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint6
   GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * (P + 1), s));
   {
     const size_t smem = (size_t)P * sizeof(uint32_t);
-    GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_pid_hist<kDigit>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most any call takes: the limit is the kernel's, not the call's
+    GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(k_pid_hist<kDigit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(sizeof(uint32_t) << kMaxPartBits)));
     int per_sm = 1;
     GBJ_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pid_hist<kDigit>, 1024, smem));
     const uint64_t grid = std::max<uint64_t>(

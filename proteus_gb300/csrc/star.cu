@@ -1059,10 +1059,15 @@ static int make_plan(gbj_ctx *ctx, const gbj_star_fact *fact, const gbj_star_dim
   }
   cudaError_t e = cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) return fail(cuda_error(ctx, e, "cudaStreamCreate"));
-  // static plus dynamic shared memory may pass 48 KB: opt in
+  // static plus dynamic shared memory may pass 48 KB: opt in, to all there is,
+  // because the limit is the kernel's and other plans have other totals
   for (auto kern : {k_star_fact<true, false>, k_star_fact<false, false>, k_star_fact<true, true>,
                     k_star_fact<false, true>}) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem.total);
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, kern);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(ctx->smem_optin - fa.sharedSizeBytes));
     if (e != cudaSuccess) return fail(cuda_error(ctx, e, "star: shared memory attribute"));
   }
   int per_sm = 1;
