@@ -371,12 +371,13 @@ __device__ __forceinline__ void load4(const int32_t *__restrict__ keys, const in
 // either the raw SoA input (items of w rows; level 1 persists across items
 // and is flushed to level 2 when the CTA finishes) or the partitioned AoS
 // pairs (one partition, or a w-row piece of one; level 1 is cleared per
-// item and a whole partition is emitted directly).  kVec: the raw columns
-// are 16-byte aligned and read 4 rows per thread per load.
+// item and a whole partition is emitted directly; a partition of up to `one`
+// rows is one item).  kVec: the raw columns are 16-byte aligned and read 4 rows
+// per thread per load.
 template <bool kPairs, bool kVec>
 __global__ void __launch_bounds__(kThreads, 2)
     k_groupby(const int32_t *__restrict__ keys, const int32_t *__restrict__ vals,
-              const int2 *__restrict__ pairs, uint64_t n, uint64_t w,
+              const int2 *__restrict__ pairs, uint64_t n, uint64_t w, uint64_t one,
               const uint64_t *__restrict__ poff, const uint64_t *__restrict__ item_off, uint32_t P,
               uint32_t tslots, uint32_t rlog, GTable g, Out o, unsigned long long *item_ctr, uint32_t *status) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -408,9 +409,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (kPairs) {
       const uint32_t a = gbjd::item_partition(item_off, P, total_items, item);
       const uint64_t p0 = poff[a], p1 = poff[a + 1];
-      lo = p0 + (item - item_off[a]) * w;
-      hi = lo + w < p1 ? lo + w : p1;
-      whole = (p1 - p0) <= w;
+      whole = p1 - p0 <= one;
+      lo = p0 + (item - item_off[a]) * w;  // item_off[a] for a whole one
+      hi = whole || lo + w > p1 ? p1 : lo + w;
     } else {
       lo = item * w;
       hi = lo + w < n ? lo + w : n;
@@ -538,30 +539,26 @@ __global__ void k_groupby_emit(GTable g, Out o, uint32_t *status) {
   }
 }
 
-// Work items of w rows per partition, as offsets, and the item counter.
+// Work items per partition, as offsets, and the item counter: one for up to
+// `one` rows, else w rows each.
 __global__ void __launch_bounds__(1024)
-    k_groupby_plan(const uint64_t *__restrict__ poff, uint32_t P, uint64_t w, uint64_t *__restrict__ items,
-                   unsigned long long *ctr) {
+    k_groupby_plan(const uint64_t *__restrict__ poff, uint32_t P, uint64_t w, uint64_t one,
+                   uint64_t *__restrict__ items, unsigned long long *ctr) {
   __shared__ uint64_t s_scan[32];
   if (threadIdx.x == 0) *ctr = 0;
-  gbjd::cta_offsets(P, [&](uint32_t p) { return (poff[p + 1] - poff[p] + w - 1) / w; }, items, s_scan);
+  gbjd::cta_offsets(P, [&](uint32_t p) -> uint64_t {
+    const uint64_t rows = poff[p + 1] - poff[p];
+    return rows <= one ? rows != 0 : (rows + w - 1) / w;
+  }, items, s_scan);
 }
 
-}  // namespace
-
-extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values,
-                           uint64_t n, const gbj_groupby_params *params, int32_t *d_out_keys,
-                           int64_t *d_out_count, int64_t *d_out_sum, int32_t *d_out_min,
-                           int32_t *d_out_max, uint64_t out_capacity, uint64_t *d_n_groups,
-                           void *stream) {
-  if (!ctx || !d_n_groups) return GBJ_ERR_INVALID;
-  if (n && (!d_keys || !d_values)) return set_error(ctx, GBJ_ERR_INVALID, "groupby: null column");
-  if (n >= (1ULL << 31)) return set_error(ctx, GBJ_ERR_INVALID, "groupby: n >= 2^31");
-  cudaStream_t s = pick_stream(ctx, stream);
-  prof_mark(ctx, s);
-  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(d_n_groups, 0, sizeof(uint64_t), s));
-  if (n == 0) return GBJ_OK;
-
+// The call itself.  `least`: with partitions, items and tables that need the
+// least memory.  Nothing is written to the output before all of its memory is
+// there.
+int groupby_impl(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values, uint64_t n,
+                 const gbj_groupby_params *params, bool least, int32_t *d_out_keys, int64_t *d_out_count,
+                 int64_t *d_out_sum, int32_t *d_out_min, int32_t *d_out_max, uint64_t out_capacity,
+                 uint64_t *d_n_groups, cudaStream_t s) {
   // ---- plan: on-chip tables for small key domains, radix partitioning
   //      (so a partition's groups fit on chip) for large ones ----
   uint64_t hint = 0;
@@ -583,9 +580,51 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
       std::max<uint64_t>(1024, hint ? std::min<uint64_t>(hint, n) : std::min<uint64_t>(n, 1ull << 24));
   if (strategy == 0) strategy = (hint && hint <= kSlots / 2) ? 1 : (hint ? 2 : 1);
 
-  Scratch scratch(ctx, s);
   // level-2 table: cap slots + 1 dedicated INT32_MIN group
-  const uint64_t cap = next_pow2(2 * groups_cap);
+  uint64_t cap = next_pow2(2 * groups_cap);
+  int bits = 1;             // strategy 2: partitions,
+  uint64_t w = 0, one = 0;  // rows of an item, and of a partition that is one item
+  uint32_t tslots_arg = kSlots, rlog_arg = 0;
+  if (strategy == 2) {
+    // Partition so each partition holds ~kSlots/4 groups.  Then add bits,
+    // without adding a partitioning pass, until a partition has 16,384 rows
+    // (4 M rows, 5000 groups: 8 bits 121 us, 6 bits 147) and is usually one work
+    // item, which is emitted directly.  One pass over 9 to 11 bits costs less
+    // than over 12, so there the items are longer instead (2^28 rows, 2^20
+    // groups: 11 bits 2840 us, 12 bits 3032).  An item has a quarter of an SM's
+    // share of the rows, so that a skewed key's rows spread over the SMs, but no
+    // fewer than 32,768, which its merge into the global table must be worth
+    // (Zipf 1.0, against items of 131,072 rows: 2^22 rows in 100,000 groups
+    // 235 -> 117 us, 2^24 in 300,000 373 -> 266).  `least`: partitions of
+    // 65,536 rows, whose tables of offsets are fewer words.
+    while (bits < kMaxPartBits && (groups_cap >> bits) > (uint64_t)kSlots / 4) ++bits;
+    const int free_bits = bits <= 8 ? 8 : bits <= 11 && !least ? 11 : kMaxPartBits;
+    const uint64_t rows = bits <= 11 && !least ? 16384 : 65536;
+    w = least ? 1u << 17
+              : std::min<uint64_t>(bits > 8 && bits <= 11 ? 1u << 18 : 1u << 17,
+                                   std::max<uint64_t>(32768, next_pow2(n / (4 * ctx->sm_count))));
+    while (bits < free_bits && (n >> bits) > rows) ++bits;
+    if (params && params->hash_bits > 0 && !hint)
+      bits = std::min(params->hash_bits, kMaxPartBits);
+    if (tuned_bits > 0) bits = std::min<int>(tuned_bits, kMaxPartBits);
+    tslots_arg = (uint32_t)std::min<uint64_t>(
+        kSlots, std::max<uint64_t>(64, next_pow2(4 * ((groups_cap + (1u << bits) - 1) >> bits))));
+    // The hint is only one: the partitions' tables take more groups than the
+    // global table is sized for, which must not depend on how items are cut.
+    // So where partitions are cut, either the global table takes whatever all
+    // of theirs can, while that is few slots, or only partitions of twice the
+    // mean rows are cut, at most half of them (2^24 rows, all cut / this rule:
+    // 100,000 groups uniform 258 / 242 us, Zipf 1.0 249 / 279; 5000 groups, with
+    // the larger table / without it, uniform 238 / 291 us, Zipf 223 / 234).
+    one = std::max(w, std::min<uint64_t>(1u << 17, 2 * (n >> bits)));
+    const uint64_t all = (uint64_t)tslots_arg << bits;
+    if (one > w && all <= (1u << 18)) {
+      one = w;
+      cap = std::max(cap, all);
+    }
+  }
+
+  Scratch scratch(ctx, s);
   GTable g;
   char *gmem;
   const uint64_t gbytes = (cap + 1) * (4 + 8 + 8 + 4 + 4) + 64;
@@ -602,13 +641,12 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
   unsigned long long *ctr;
   GBJ_TRY(scratch.get(1, &ctr));
 
-  uint32_t tslots_arg = kSlots, rlog_arg = 0;
   // as many accumulator columns (up to 16) as the table budget allows
   auto pick_rlog = [&]() {
     rlog_arg = 0;
     while (rlog_arg < 4 && (size_t)tslots_arg * slot_bytes(rlog_arg + 1) <= kTableBudget) ++rlog_arg;
   };
-  auto launch = [&](auto kern, int tab, const int2 *pairs, uint64_t w, const uint64_t *poff,
+  auto launch = [&](auto kern, int tab, const int2 *pairs, uint64_t w, uint64_t one, const uint64_t *poff,
                     const uint64_t *items, uint32_t P) -> int {
     const size_t smem = (size_t)tab * slot_bytes(rlog_arg);
     // the most any call takes: the limit is the kernel's, not the call's
@@ -616,7 +654,7 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
     int per_sm = 1;
     GBJ_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
     per_sm = std::max(per_sm, 1);
-    kern<<<ctx->sm_count * per_sm, kThreads, smem, s>>>(d_keys, d_values, pairs, n, w, poff, items,
+    kern<<<ctx->sm_count * per_sm, kThreads, smem, s>>>(d_keys, d_values, pairs, n, w, one, poff, items,
                                                         P, tslots_arg, rlog_arg, g, o, ctr, ctx->d_status);
     return after_launch(ctx, "k_groupby", s);
   };
@@ -632,33 +670,10 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
     tslots_arg = (uint32_t)std::min<uint64_t>(kSlots, std::max<uint64_t>(64, next_pow2(16 * (hint ? hint : groups_cap))));
     pick_rlog();
     const bool aligned = (reinterpret_cast<uintptr_t>(d_keys) | reinterpret_cast<uintptr_t>(d_values)) % 16 == 0;
-    if (aligned) GBJ_TRY(launch(k_groupby<false, true>, (int)tslots_arg, nullptr, wq, nullptr, nullptr, 0));
-    else GBJ_TRY(launch(k_groupby<false, false>, (int)tslots_arg, nullptr, wq, nullptr, nullptr, 0));
+    if (aligned) GBJ_TRY(launch(k_groupby<false, true>, (int)tslots_arg, nullptr, wq, 0, nullptr, nullptr, 0));
+    else GBJ_TRY(launch(k_groupby<false, false>, (int)tslots_arg, nullptr, wq, 0, nullptr, nullptr, 0));
   } else {
-    // Partition so each partition holds ~kSlots/4 groups.  Then add bits,
-    // without adding a partitioning pass, until a partition has 16,384 rows
-    // (4 M rows, 5000 groups: 8 bits 121 us, 6 bits 147) and is usually one work
-    // item, which is emitted directly.  One pass over 9 to 11 bits costs less
-    // than over 12, so there the items are longer instead (2^28 rows, 2^20
-    // groups: 11 bits 2840 us, 12 bits 3032).  An item has a quarter of an SM's
-    // share of the rows, so that a skewed key's rows spread over the SMs, but no
-    // fewer than 32,768, which its merge into the global table must be worth
-    // (Zipf 1.0, against items of 131,072 rows: 2^22 rows in 100,000 groups
-    // 235 -> 117 us, 2^24 in 300,000 373 -> 266; uniform 2^24 in 100,000, where
-    // partitions are now two items, 212 -> 225).
-    int bits = 1;
-    while (bits < kMaxPartBits && (groups_cap >> bits) > (uint64_t)kSlots / 4) ++bits;
-    const int free_bits = bits <= 8 ? 8 : bits <= 11 ? 11 : kMaxPartBits;
-    const uint64_t rows = bits <= 11 ? 16384 : 65536;
-    const uint64_t w = std::min<uint64_t>(bits > 8 && bits <= 11 ? 1u << 18 : 1u << 17,
-                                          std::max<uint64_t>(32768, next_pow2(n / (4 * ctx->sm_count))));
-    while (bits < free_bits && (n >> bits) > rows) ++bits;
-    if (params && params->hash_bits > 0 && strategy == 2 && !hint)
-      bits = std::min(params->hash_bits, kMaxPartBits);
-    if (tuned_bits > 0) bits = std::min<int>(tuned_bits, kMaxPartBits);
     const uint32_t P = 1u << bits;
-    tslots_arg = (uint32_t)std::min<uint64_t>(
-        kSlots, std::max<uint64_t>(64, next_pow2(4 * ((groups_cap + P - 1) >> bits))));
     pick_rlog();
     int2 *pairs;
     uint64_t *poff, *items;
@@ -667,13 +682,34 @@ extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d
     GBJ_TRY(scratch.get(P + 1, &items));
     GBJ_TRY(partition_tuples(ctx, d_keys, d_values, n, GBJ_DIGIT_HASH, 0, bits, pairs, nullptr,
                              nullptr, poff, s));
-    k_groupby_plan<<<1, 1024, 0, s>>>(poff, P, w, items, ctr);
+    k_groupby_plan<<<1, 1024, 0, s>>>(poff, P, w, one, items, ctr);
     GBJ_TRY(after_launch(ctx, "k_groupby_plan", s));
-    GBJ_TRY(launch(k_groupby<true, false>, (int)tslots_arg, pairs, w, poff, items, P));
+    GBJ_TRY(launch(k_groupby<true, false>, (int)tslots_arg, pairs, w, one, poff, items, P));
   }
   const uint64_t emit_threads = 256;
   const uint64_t emit_blocks =
       std::min<uint64_t>((cap + emit_threads) / emit_threads, (uint64_t)ctx->sm_count * 8);
   k_groupby_emit<<<(unsigned)emit_blocks, emit_threads, 0, s>>>(g, o, ctx->d_status);
   return after_launch(ctx, "k_groupby_emit", s);
+}
+
+}  // namespace
+
+extern "C" int gbj_groupby(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values,
+                           uint64_t n, const gbj_groupby_params *params, int32_t *d_out_keys,
+                           int64_t *d_out_count, int64_t *d_out_sum, int32_t *d_out_min,
+                           int32_t *d_out_max, uint64_t out_capacity, uint64_t *d_n_groups,
+                           void *stream) {
+  if (!ctx || !d_n_groups) return GBJ_ERR_INVALID;
+  if (n && (!d_keys || !d_values)) return set_error(ctx, GBJ_ERR_INVALID, "groupby: null column");
+  if (n >= (1ULL << 31)) return set_error(ctx, GBJ_ERR_INVALID, "groupby: n >= 2^31");
+  cudaStream_t s = pick_stream(ctx, stream);
+  prof_mark(ctx, s);
+  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(d_n_groups, 0, sizeof(uint64_t), s));
+  if (n == 0) return GBJ_OK;
+  const int rc = groupby_impl(ctx, d_keys, d_values, n, params, false, d_out_keys, d_out_count, d_out_sum, d_out_min,
+                              d_out_max, out_capacity, d_n_groups, s);
+  if (rc != GBJ_ERR_OOM) return rc;
+  return groupby_impl(ctx, d_keys, d_values, n, params, true, d_out_keys, d_out_count, d_out_sum, d_out_min, d_out_max,
+                      out_capacity, d_n_groups, s);
 }
