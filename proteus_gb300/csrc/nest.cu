@@ -47,16 +47,17 @@ __device__ __forceinline__ uint64_t fmix64(uint64_t k) {  // murmur3 64-bit fina
 // arrays: a load of a sector that takes atomics waits for them in L2.
 // Measured on GB300, 2^17 slots (record load and both additions, G rows/s):
 // five arrays 33; one 32-byte record with sum and count in it 62; two arrays
-// 103.  2^22 slots (past L2): one record 53, two arrays 40.
+// 103.  2^22 slots (past L2): one record 53, two arrays 40.  A pool without
+// room for 48 bytes a slot gets 40: the count is then the record's fourth word.
 struct Table64 {
-  unsigned long long *rec, *acc;
+  unsigned long long *rec, *sums, *cnts;
   uint64_t mask;  // slots - 1; slot mask + 1 is INT64_MIN's
-  bool vals;
-  __device__ __forceinline__ unsigned long long *key(uint64_t s) const { return rec + (vals ? 4 * s : s); }
+  uint32_t rec_shift, sum_shift, cnt_shift;  // log2 of the words from one slot's to the next
+  __device__ __forceinline__ unsigned long long *key(uint64_t s) const { return rec + (s << rec_shift); }
   __device__ __forceinline__ unsigned long long *mn(uint64_t s) const { return rec + 4 * s + 1; }
   __device__ __forceinline__ unsigned long long *mx(uint64_t s) const { return rec + 4 * s + 2; }
-  __device__ __forceinline__ unsigned long long *sum(uint64_t s) const { return acc + 2 * s; }
-  __device__ __forceinline__ unsigned long long *cnt(uint64_t s) const { return acc + (vals ? 2 * s + 1 : s); }
+  __device__ __forceinline__ unsigned long long *sum(uint64_t s) const { return sums + (s << sum_shift); }
+  __device__ __forceinline__ unsigned long long *cnt(uint64_t s) const { return cnts + (s << cnt_shift); }
 };
 
 struct Rec64 {
@@ -158,6 +159,9 @@ __global__ void __launch_bounds__(kThreads)
     if (kVals) return ld_rec(t.key(h));
     return Rec64{*(volatile unsigned long long *)t.key(h), 0, 0, 0};
   };
+  // even lanes add to sums, odd ones to counts
+  unsigned long long *const lane_acc = lane & 1 ? t.cnts : t.sums;
+  const uint32_t lane_shift = lane & 1 ? t.cnt_shift : t.sum_shift;
   // a row into slot s (all lanes call it; s < 0: nothing to do)
   auto add = [&](int64_t s, int64_t v, const Rec64 &e) {
     if (kVals) {
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(kThreads)
       for (int half = 0; half < 2; ++half) {
         const int from = (lane >> 1) + 16 * half;
         const int64_t fs = __shfl_sync(0xffffffffu, s, from), fv = __shfl_sync(0xffffffffu, v, from);
-        if (fs >= 0) atomicAdd(t.sum((uint64_t)fs) + (lane & 1), lane & 1 ? 1ull : (unsigned long long)fv);
+        if (fs >= 0) atomicAdd(lane_acc + ((uint64_t)fs << lane_shift), lane & 1 ? 1ull : (unsigned long long)fv);
       }
     } else if (s >= 0) {
       atomicAdd(t.cnt((uint64_t)s), 1ull);
@@ -541,15 +545,16 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Table64 with `slots` slots (+ the INT64_MIN slot), zeroed, from scratch.
-int make_table(gbj_ctx *ctx, Scratch &scratch, uint64_t slots, bool with_vals, cudaStream_t s, Table64 *t) {
-  const uint64_t cols = with_vals ? 6 : 2;  // record 4 + pair 2, or key + count
+// `words` of a slot: 6 (record, {sum, count}) or 5 (record with the count, sum)
+// with values, 2 (key, count) without.
+int make_table(gbj_ctx *ctx, Scratch &scratch, uint64_t slots, uint32_t words, cudaStream_t s, Table64 *t) {
   unsigned long long *mem;
-  GBJ_TRY(scratch.get(cols * (slots + 1), &mem));  // pool blocks are 256-byte aligned: 32-byte records
-  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(mem, 0, sizeof(unsigned long long) * cols * (slots + 1), s));
-  t->rec = mem;
-  t->acc = mem + (with_vals ? 4 : 1) * (slots + 1);
-  t->mask = slots - 1;
-  t->vals = with_vals;
+  GBJ_TRY(scratch.get(words * (slots + 1), &mem));  // pool blocks are 256-byte aligned: 32-byte records
+  GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(mem, 0, sizeof(unsigned long long) * words * (slots + 1), s));
+  unsigned long long *const rest = mem + (words == 2 ? 1 : 4) * (slots + 1);
+  if (words == 6) *t = {mem, rest, rest + 1, slots - 1, 2, 1, 1};
+  else if (words == 5) *t = {mem, rest, mem + 3, slots - 1, 2, 0, 2};
+  else *t = {mem, nullptr, rest, slots - 1, 0, 0, 0};
   return GBJ_OK;
 }
 
@@ -580,8 +585,12 @@ int nest_impl(gbj_ctx *ctx, const int64_t *d_keys, const V *d_vals, uint64_t n, 
   uint64_t slots = limit;
   if (!use_l1)
     while (slots < 4 * limit && 2 * slots * per_slot <= (32ull << 20) && (slots == limit || 16 * slots <= n)) slots *= 2;
-  int rc = make_table(ctx, scratch, slots, d_vals != nullptr, s, &t);
-  if (rc == GBJ_ERR_OOM && slots > limit) rc = make_table(ctx, scratch, limit, d_vals != nullptr, s, &t);
+  unsigned long long *ctr = nullptr;
+  if (use_l1) GBJ_TRY(scratch.get(1, &ctr));
+  // a pool without room for it: the fewest slots, then the fewest bytes of one
+  int rc = make_table(ctx, scratch, slots, d_vals ? 6 : 2, s, &t);
+  if (rc == GBJ_ERR_OOM && slots > limit) rc = make_table(ctx, scratch, limit, d_vals ? 6 : 2, s, &t);
+  if (rc == GBJ_ERR_OOM && d_vals) rc = make_table(ctx, scratch, limit, 5, s, &t);
   if (rc) return rc;
   if (use_l1) {
     // few groups: the on-chip level first (tables at 8 x groups)
@@ -590,8 +599,6 @@ int nest_impl(gbj_ctx *ctx, const int64_t *d_keys, const V *d_vals, uint64_t n, 
     uint32_t rlog = 0;  // as many accumulator columns (<= 32) as the budget allows
     while (rlog < 5 && (size_t)tslots * l1_slot_bytes(rlog + 1) <= kL1Budget) ++rlog;
     const size_t smem = (size_t)tslots * l1_slot_bytes(rlog);
-    unsigned long long *ctr;
-    GBJ_TRY(scratch.get(1, &ctr));
     GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
     auto kern = k_nest_l1<V>;
     // the most any call takes: the limit is the kernel's, not the call's
@@ -676,7 +683,7 @@ extern "C" int gbj_radix_join_count_i64(gbj_ctx *ctx, const int64_t *d_r_keys, u
   if (nr == 0 || ns == 0) return GBJ_OK;
   Scratch scratch(ctx, s);
   Table64 t;
-  GBJ_TRY(make_table(ctx, scratch, next_pow2(std::max<uint64_t>(2 * nr, 1024)), false, s, &t));
+  GBJ_TRY(make_table(ctx, scratch, next_pow2(std::max<uint64_t>(2 * nr, 1024)), 2, s, &t));
   k_nest_build<int64_t, false><<<grid_for(ctx, nr), kThreads, 0, s>>>(d_r_keys, nullptr, nr, t, ctx->d_status);
   GBJ_TRY(after_launch(ctx, "k_nest_build", s));
   k_join_count_probe<<<grid_for(ctx, ns), kThreads, 0, s>>>(d_s_keys, ns, t,
