@@ -144,9 +144,13 @@ struct NestQueue {
 // probing on where it was found, a warp would wait for the longest of 32
 // chains, an L2 round trip a slot.  Measured, 2^27 rows of int64 keys and
 // values, 2^16 groups: 3.93 ms before, 1.22 ms now.
+//
+// `limit`: the groups that the table may take.  A row that has passed as many
+// slots with other keys is one too many, however many slots there are (2^20
+// groups in a table for 8192 that has 32,768 slots: refused in 46 ms, not 183).
 template <typename V, bool kVals>
 __global__ void __launch_bounds__(kThreads)
-    k_nest_build(const int64_t *__restrict__ keys, const V *__restrict__ vals, uint64_t n, Table64 t,
+    k_nest_build(const int64_t *__restrict__ keys, const V *__restrict__ vals, uint64_t n, Table64 t, uint64_t limit,
                  uint32_t *status) {
   constexpr int kRows = 2;
   __shared__ NestQueue s_q[kThreads / 32];
@@ -241,7 +245,7 @@ __global__ void __launch_bounds__(kThreads)
     for (int u = 0; u < kRows; ++u) {
       const bool here = e[u].key == ((unsigned long long)k[u] ^ kFlip64);
       add(ok[u] && here ? (int64_t)h[u] : -1, v[u], e[u]);
-      push(ok[u] && !here, k[u], v[u], e[u].key == 0 ? h[u] : (h[u] + 1) & t.mask, t.mask);
+      push(ok[u] && !here, k[u], v[u], e[u].key == 0 ? h[u] : (h[u] + 1) & t.mask, limit);
       while (qn >= 32) step(32);
     }
   }
@@ -609,8 +613,8 @@ int nest_impl(gbj_ctx *ctx, const int64_t *d_keys, const V *d_vals, uint64_t n, 
     kern<<<ctx->sm_count * per_sm, kL1Threads, smem, s>>>(d_keys, d_vals, n, tslots, rlog, t, ctr, ctx->d_status);
     GBJ_TRY(after_launch(ctx, "k_nest_l1", s));
   } else {
-    if (d_vals) k_nest_build<V, true><<<grid_for(ctx, n), kThreads, 0, s>>>(d_keys, d_vals, n, t, ctx->d_status);
-    else k_nest_build<V, false><<<grid_for(ctx, n), kThreads, 0, s>>>(d_keys, d_vals, n, t, ctx->d_status);
+    if (d_vals) k_nest_build<V, true><<<grid_for(ctx, n), kThreads, 0, s>>>(d_keys, d_vals, n, t, limit, ctx->d_status);
+    else k_nest_build<V, false><<<grid_for(ctx, n), kThreads, 0, s>>>(d_keys, d_vals, n, t, limit, ctx->d_status);
     GBJ_TRY(after_launch(ctx, "k_nest_build", s));
   }
   k_nest_emit<M><<<grid_for(ctx, t.mask + 2), kThreads, 0, s>>>(
@@ -684,7 +688,7 @@ extern "C" int gbj_radix_join_count_i64(gbj_ctx *ctx, const int64_t *d_r_keys, u
   Scratch scratch(ctx, s);
   Table64 t;
   GBJ_TRY(make_table(ctx, scratch, next_pow2(std::max<uint64_t>(2 * nr, 1024)), 2, s, &t));
-  k_nest_build<int64_t, false><<<grid_for(ctx, nr), kThreads, 0, s>>>(d_r_keys, nullptr, nr, t, ctx->d_status);
+  k_nest_build<int64_t, false><<<grid_for(ctx, nr), kThreads, 0, s>>>(d_r_keys, nullptr, nr, t, t.mask, ctx->d_status);
   GBJ_TRY(after_launch(ctx, "k_nest_build", s));
   k_join_count_probe<<<grid_for(ctx, ns), kThreads, 0, s>>>(d_s_keys, ns, t,
                                                             reinterpret_cast<unsigned long long *>(d_count));
