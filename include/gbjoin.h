@@ -205,7 +205,8 @@ uint64_t gbj_table_slots(const gbj_table *table);
  * counting-sort cluster of radix_cluster_nopadding.
  * d_payload may be NULL: then the 0-based row position is carried instead.
  * d_offsets receives 2^bits + 1 partition start offsets.  bits in [1, 15],
- * shift + bits <= 32, n < 2^31.  No host synchronisation. */
+ * shift + bits <= 32, n < 2^31.  From 9 bits on the output columns may overlap
+ * the input columns (not each other).  No host synchronisation. */
 typedef enum gbj_digit { GBJ_DIGIT_KEY = 0, GBJ_DIGIT_HASH = 1 } gbj_digit;
 
 int gbj_partition(gbj_ctx *ctx, const int32_t *d_keys,

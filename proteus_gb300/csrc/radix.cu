@@ -1063,7 +1063,15 @@ int partition_impl(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals, uint6
   constexpr int kPass = kHashOut ? kDigitPre : kDigit;
   const uint32_t P = 1u << bits, pmask = P - 1;
   Scratch scratch(ctx, s);
-  const bool wide = passes == 0 && bits > 8 && bits <= kWideBits;
+  // one pass writes the output while it still reads the columns, two passes do
+  // not: columns that are partitioned in place take two from 9 bits on
+  auto apart = [&](const void *in, const void *out) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(in), b = reinterpret_cast<uintptr_t>(out);
+    return !in || !out || a + 4 * n <= b || b + 4 * n <= a;
+  };
+  const bool in_place = !out_pairs && !(apart(keys, out_keys) && apart(keys, out_vals) && apart(vals, out_keys) &&
+                                        apart(vals, out_vals));
+  const bool wide = passes == 0 && bits > 8 && bits <= kWideBits && !in_place;
   const bool one = wide || passes == 1 || (passes == 0 && bits <= 8);
   const int bits2 = bits / 2, bits1 = bits - bits2;
   const uint32_t B1 = 1u << bits1, m2 = (1u << bits2) - 1;
