@@ -609,9 +609,10 @@ int gbj_server_unregister_table(gbj_server *srv, uint64_t table_id);
  * Later calls of that shape that pass no explicit sizing use it:
  *   radix join     join kernel block size (512: two blocks per SM with
  *                  4608-tuple build chunks; 1024: one block, 9216) and,
- *                  for each, partition bits 1..15 (bits > 8 means two
- *                  passes) -- gbj_radix_join_agg with params NULL or zero
- *                  bits / block;
+ *                  for each, partition bits around those of the untuned plan
+ *                  and of the fewest partitions that fit (up to 12 bits are
+ *                  one pass, more are two) -- gbj_radix_join_agg with params
+ *                  NULL or zero bits / block;
  *   plain join     table size 2^hash_bits (load factor 1/2, 1/4, 1/8) --
  *                  gbj_join_build with hash_bits 0;
  *   group-by       strategy 1, or strategy 2 with its partition bits --

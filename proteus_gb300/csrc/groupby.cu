@@ -586,24 +586,17 @@ int groupby_impl(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values, u
   uint64_t w = 0, one = 0;  // rows of an item, and of a partition that is one item
   uint32_t tslots_arg = kSlots, rlog_arg = 0;
   if (strategy == 2) {
-    // Partition so each partition holds ~kSlots/4 groups.  Then add bits,
-    // without adding a partitioning pass, until a partition has 16,384 rows
-    // (4 M rows, 5000 groups: 8 bits 121 us, 6 bits 147) and is usually one work
-    // item, which is emitted directly.  One pass over 9 to 11 bits costs less
-    // than over 12, so there the items are longer instead (2^28 rows, 2^20
-    // groups: 11 bits 2840 us, 12 bits 3032).  An item has a quarter of an SM's
-    // share of the rows, so that a skewed key's rows spread over the SMs, but no
-    // fewer than 32,768, which its merge into the global table must be worth
-    // (Zipf 1.0, against items of 131,072 rows: 2^22 rows in 100,000 groups
-    // 235 -> 117 us, 2^24 in 300,000 373 -> 266).  `least`: partitions of
-    // 65,536 rows, whose tables of offsets are fewer words.
-    while (bits < kMaxPartBits && (groups_cap >> bits) > (uint64_t)kSlots / 4) ++bits;
-    const int free_bits = bits <= 8 ? 8 : bits <= 11 && !least ? 11 : kMaxPartBits;
-    const uint64_t rows = bits <= 11 && !least ? 16384 : 65536;
+    // A partition holds about kSlots / 4 groups (auto_plan.h).  An item has a
+    // quarter of an SM's share of the rows, so that a skewed key's rows spread
+    // over the SMs, but no fewer than 32,768, which its merge into the global
+    // table must be worth (Zipf 1.0, against items of 131,072 rows: 2^22 rows in
+    // 100,000 groups 235 -> 117 us, 2^24 in 300,000 373 -> 266).
+    static_assert(kSlots == 4096, "groupby_fit_bits");
+    const int fit = groupby_fit_bits(groups_cap);
     w = least ? 1u << 17
-              : std::min<uint64_t>(bits > 8 && bits <= 11 ? 1u << 18 : 1u << 17,
+              : std::min<uint64_t>(fit > 8 && fit <= 11 ? 1u << 18 : 1u << 17,
                                    std::max<uint64_t>(32768, next_pow2(n / (4 * ctx->sm_count))));
-    while (bits < free_bits && (n >> bits) > rows) ++bits;
+    bits = groupby_auto_bits(n, groups_cap, least);
     if (params && params->hash_bits > 0 && !hint)
       bits = std::min(params->hash_bits, kMaxPartBits);
     if (tuned_bits > 0) bits = std::min<int>(tuned_bits, kMaxPartBits);

@@ -34,8 +34,8 @@
 //    load.  The partition that INT32_MIN (the empty marker) hashes to uses
 //    an index table instead.
 #include <algorithm>
-#include <cmath>
 
+#include "auto_plan.h"
 #include "gbj_internal.cuh"
 #include "radix.cuh"
 #include "scan.cuh"
@@ -960,15 +960,6 @@ int launch_join(gbj_ctx *ctx, const int2 *R, const uint64_t *ro, const int2 *S,
   return after_launch(ctx, "k_radix_join", s);
 }
 
-// The two join kernel shapes: 1024 threads with build chunks of 9216 tuples
-// (one block per SM), or 512 threads with chunks of 4608 (two blocks per
-// SM; partitions then need one more radix bit).
-struct JoinShape {
-  int threads, rmax;
-};
-constexpr JoinShape kJoinWide{1024, 9216};
-constexpr JoinShape kJoinPair{512, 4608};
-
 template <int kRMax, int kThreads, int kCtas>
 int launch_join_agg(gbj_ctx *ctx, bool by_rows, const AggSpec &spec, const int2 *R, const uint64_t *ro,
                     const int2 *S, const uint64_t *so, const uint64_t *items, uint32_t P, uint32_t w,
@@ -1226,31 +1217,11 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
   if (n_build == 0 || n_probe == 0) return init_agg_out(ctx, spec, d_out, s);
 
   // ---- plan: the fewest radix bits whose largest expected build partition
-  //      (mean + 5 sd) fits the on-chip table, but enough partitions to give
-  //      every CTA a few work items; explicit params override ----
+  //      fits the on-chip table, but enough partitions to give every CTA a few
+  //      work items (auto_plan.h); explicit params override ----
   const int passes = params ? params->passes : 0;
-  auto fit_bits = [&](int rmax) {
-    int b = 1;
-    while (b < kMaxPartBits) {
-      const double mean = (double)n_build / (double)(1u << b);
-      if (mean + 5.0 * std::sqrt(mean) <= (double)rmax) break;
-      ++b;
-    }
-    return b;
-  };
-  // 256 to 1024 partitions of about 2^14 tuples of both sides: fewer leave
-  // SMs without work (2^16 and 2^20 rows: 4 bits 219 us, 8 bits 69), more
-  // cost a table set-up of 4 us each (12 bits at 2^20 and 2^24 rows 260 us, 10
-  // bits 200, 8 bits 316)
-  const int even = std::max(8, std::min(10, log2_ceil((n_build + n_probe) >> 14)));
-  // Join kernel shape: the caller's block size, else an autotuned one, else
-  // two 512-thread blocks per SM while its partitions are small enough at 10
-  // bits, else 1024 threads, which take twice the tuples and so one radix bit
-  // less (us; 4 M and 128 M rows: 512 threads at 10 bits 1144, at 11 bits
-  // 1076, 1024 threads at 10 bits 1080; 16 M and 64 M: 512 at 12 bits 799,
-  // 1024 at 11 bits 752; 30 M and 128 M: 512 at 13 bits, two passes, 1758,
-  // 1024 at 12 bits 1478; 2^27 and 2^29: 15 bits 7631, 14 bits 7162).
-  constexpr int kPairRoom = 3900;  // a fuller 512-thread table loses more than a bit costs
+  // Join kernel shape: the caller's block size, else an autotuned one, else by
+  // the sizes (auto_plan.h).
   const bool explicit_bits = params && (params->log_parts > 0 || params->bits > 0);
   int block = params ? params->block : 0;
   if (!block) {
@@ -1259,14 +1230,14 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
       block = tb;
     } else if (explicit_bits) {
       const int b = params->bits > 0 ? params->bits : params->log_parts;
-      block = fit_bits(kJoinPair.rmax) <= b ? kJoinPair.threads : kJoinWide.threads;
+      block = radix_fit_bits(n_build, kJoinPair.rmax) <= b ? kJoinPair.threads : kJoinWide.threads;
     } else {
-      block = std::max(fit_bits(kPairRoom), even) <= 10 ? kJoinPair.threads : kJoinWide.threads;
+      block = radix_auto_threads(n_build, n_probe);
     }
   }
   const JoinShape shape = block == kJoinWide.threads ? kJoinWide : kJoinPair;
   const uint32_t kRMax = (uint32_t)shape.rmax;
-  int bits = std::max(even, fit_bits(shape.threads == kJoinPair.threads ? kPairRoom : shape.rmax));
+  int bits = radix_auto_bits(n_build, n_probe, shape.threads);
   if (!explicit_bits) {  // an autotuned choice for this size bucket, if any
     const int32_t tb = tuned_value(ctx, tune_key(shape.threads == kJoinWide.threads ? "radix" : "radix512",
                                                  n_build, n_probe));

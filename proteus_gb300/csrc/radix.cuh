@@ -1,10 +1,9 @@
 // Radix partitioning shared by the partitioned join and group-by.
 #pragma once
+#include "auto_plan.h"
 #include "gbj_internal.cuh"
 
 namespace gbj {
-
-constexpr int kMaxPartBits = 15;
 
 // Partitions n (key, value) tuples on digit = (f(key) >> shift) & (2^bits-1)
 // into a contiguous, partition-major output.  vals == nullptr carries the

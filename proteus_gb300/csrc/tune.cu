@@ -12,13 +12,13 @@
 // relbuilder.cpp:653-668) and fixes its radix bits at compile time
 // (NUM_RADIX_BITS, core/platform/lib/util/radix/joins/radix-join.cpp).
 #include <algorithm>
-#include <cmath>
 #include <cstdio>
 #include <fstream>
 #include <functional>
 #include <sstream>
 #include <vector>
 
+#include "auto_plan.h"
 #include "gbj_internal.cuh"
 
 using namespace gbj;
@@ -99,20 +99,15 @@ extern "C" int gbj_autotune_radix_join(gbj_ctx *ctx, const int32_t *d_build_keys
   cudaStream_t s = pick_stream(ctx, stream);
   int64_t *out = nullptr;
   GBJ_TRY(pool_alloc(ctx, GBJ_MAX_AGGS * sizeof(int64_t), s, reinterpret_cast<void **>(&out)));
-  // both join kernel shapes (512 threads, two blocks per SM, chunks of 4608
-  // build tuples; 1024 threads, one block, chunks of 9216), each with the
-  // radix bits around its default: fewest bits whose mean partition fits
+  // both join kernel shapes, each with the radix bits around those of the
+  // untuned plan and of the fewest partitions (auto_plan.h)
   const std::string kblock = tune_key("radixblock", n_build, n_probe);
   const int32_t prev_block = tuned_value(ctx, kblock);
   int rc = GBJ_OK;
   int32_t best_block = -1, best_b = -1;
   double best_t = 1e30;
-  for (const int32_t block : {512, 1024}) {
-    const double rmax = block == 1024 ? 9216.0 : 4608.0;
-    int d = 1;
-    while (d < 15 && (double)n_build / (double)(1u << d) > rmax) ++d;
-    std::vector<int32_t> cands;
-    for (int b = std::max(1, d - 2); b <= std::min(15, d + 2); ++b) cands.push_back(b);
+  for (const int32_t block : {kJoinPair.threads, kJoinWide.threads}) {
+    const std::vector<int32_t> cands = radix_candidates(n_build, n_probe, block);
     set_tuned(ctx, kblock, block);
     int32_t bits = -1;
     double t = 0;
@@ -164,12 +159,11 @@ extern "C" int gbj_autotune_groupby(gbj_ctx *ctx, const int32_t *d_keys, const i
   if (n == 0 || expected_groups == 0)
     return set_error(ctx, GBJ_ERR_INVALID, "autotune: empty input or unknown group count");
   cudaStream_t s = pick_stream(ctx, stream);
-  // strategy 1 (on-chip + global table) and strategy 2 around its default bits
-  const uint64_t groups_cap = std::max<uint64_t>(1024, std::min<uint64_t>(expected_groups, n));
-  int d = 1;
-  while (d < 15 && (groups_cap >> d) > 1024) ++d;
+  // strategy 1 (on-chip + global table), and strategy 2 with the bits around
+  // those of the untuned plan and of the fewest partitions
   std::vector<int32_t> cands = {(1 << 8) | 0};
-  for (int b = std::max(1, d - 1); b <= std::min(15, d + 2); ++b) cands.push_back((2 << 8) | b);
+  for (int b : groupby_candidates(n, std::max<uint64_t>(1024, std::min<uint64_t>(expected_groups, n))))
+    cands.push_back((2 << 8) | b);
   const uint64_t cap = std::min<uint64_t>(n, expected_groups) + 16;
   char *mem = nullptr;
   const uint64_t bytes = cap * (4 + 8 + 8 + 4 + 4) + 64;
