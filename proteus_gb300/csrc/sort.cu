@@ -197,24 +197,20 @@ constexpr int kThreads = 512;
 constexpr int kSmallItems = 4, kBigItems = 12;  // rows per thread
 constexpr int kWarps = kThreads / 32;
 
-// What the passes do, worked out on the device by the histogram's last CTA.
-struct SortPlan {
-  uint32_t base[4][kRadix];  // rows with a smaller digit
-  int32_t src[4], dst[4];    // buffer a pass reads / writes: 0, 1; -1 the columns; src -2: the digit is skipped
-};
-
+// The digits' counts, and what the passes do, worked out on the device by the
+// histogram's last CTA.
 struct SortState {
-  uint32_t hist[4][kRadix];
+  uint32_t hist[4][kRadix];  // rows with the digit, then rows with a smaller one
   uint32_t done;
-  uint32_t ticket[4];  // the passes' next tile
+  uint32_t ticket[4];      // the passes' next tile
+  int32_t src[4], dst[4];  // buffer a pass reads / writes: 0, 1; -1 the columns; src -2: the digit is skipped
   uint32_t pad[3];
 };
 
 constexpr int kHistThreads = 512;
 
 __global__ void __launch_bounds__(kHistThreads)
-    k_sort_hist(const int32_t *__restrict__ keys, uint32_t n, uint32_t flip, SortState *__restrict__ st,
-                SortPlan *__restrict__ plan) {
+    k_sort_hist(const int32_t *__restrict__ keys, uint32_t n, uint32_t flip, SortState *__restrict__ st) {
   __shared__ uint32_t h[4][kRadix];
   __shared__ uint32_t s_last, s_triv[4], wsum[32];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -265,7 +261,7 @@ __global__ void __launch_bounds__(kHistThreads)
     __syncthreads();
     uint32_t s = incl - x;
     for (int w = (tid >> 8) * 8; w < (tid >> 5); ++w) s += wsum[w];
-    plan->base[p][d] = s;
+    st->hist[p][d] = s;  // this thread read it above
     __syncthreads();
   }
   if (tid == 0) {
@@ -275,10 +271,10 @@ __global__ void __launch_bounds__(kHistThreads)
     while (s_triv[last]) --last;
     int at = -1;  // where the rows are
     for (int p = 0; p < 4; ++p) {
-      plan->src[p] = s_triv[p] ? -2 : at;
+      st->src[p] = s_triv[p] ? -2 : at;
       if (s_triv[p]) continue;
       at = p == last ? -1 : at == 0 ? 1 : 0;
-      plan->dst[p] = at;
+      st->dst[p] = at;
     }
   }
 }
@@ -301,17 +297,17 @@ __device__ __forceinline__ void st_status(W *p, W v) {
 
 template <int kItems, typename W>
 __global__ void __launch_bounds__(kThreads, 2)
-    k_sort_pass(Cols c, uint32_t n, int pass, const SortPlan *__restrict__ plan, SortState *__restrict__ st,
-                uint32_t *__restrict__ k0, uint32_t *__restrict__ v0, uint32_t *__restrict__ k1,
-                uint32_t *__restrict__ v1, W *__restrict__ status, uint32_t *dev_status) {
+    k_sort_pass(Cols c, uint32_t n, int pass, SortState *__restrict__ st, uint32_t *__restrict__ k0,
+                uint32_t *__restrict__ v0, uint32_t *__restrict__ k1, uint32_t *__restrict__ v1,
+                W *__restrict__ status, uint32_t *dev_status) {
   constexpr uint32_t kTile = kThreads * kItems;
   extern __shared__ __align__(16) unsigned char smem[];
   RankSmem<kWarps> &S = *reinterpret_cast<RankSmem<kWarps> *>(smem);
   uint32_t *sk = reinterpret_cast<uint32_t *>(smem + sizeof(RankSmem<kWarps>)), *sv = sk + kTile;
   __shared__ uint32_t s_tile, s_out[kRadix];
-  const int src = plan->src[pass];
+  const int src = st->src[pass];
   if (src == -2) return;
-  const int dst = plan->dst[pass];
+  const int dst = st->dst[pass];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, shift = 8 * pass;
   if (tid == 0) s_tile = atomicAdd(&st->ticket[pass], 1u);
   __syncthreads();
@@ -377,7 +373,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       p -= got * kRadix;
     }
     if (tile) st_status<W>(mine + tid, ok ? ((W)(before + tot) << 2) | kUpTo : (W)kGaveUp);
-    s_out[tid] = plan->base[pass][tid] + before - S.start[tid];
+    s_out[tid] = st->hist[pass][tid] + before - S.start[tid];
   }
   if (__syncthreads_or(!ok)) {  // a predecessor never published: report and stop
     if (tid == 0) gbjd::latch(dev_status, GBJ_DEV_TIMEOUT);
@@ -415,23 +411,21 @@ int sort_tiles(gbj_ctx *ctx, const Cols &c, uint32_t n, cudaStream_t s) {
   const uint32_t ntiles = (n + kTile - 1) / kTile;
   Scratch scratch(ctx, s);
   uint32_t *buf;
-  SortPlan *plan;
   char *zero;  // counters and the passes' status words, cleared together
   const uint64_t words = (uint64_t)ntiles * kRadix, zbytes = sizeof(SortState) + 4 * words * sizeof(W);
   GBJ_TRY(scratch.get(4 * (uint64_t)n, &buf));
-  GBJ_TRY(scratch.get(1, &plan));
   GBJ_TRY(scratch.get(zbytes, &zero));
   GBJ_CHECK_CUDA(ctx, cudaMemsetAsync(zero, 0, zbytes, s));
   SortState *st = reinterpret_cast<SortState *>(zero);
   W *status = reinterpret_cast<W *>(zero + sizeof(SortState));
   const unsigned hgrid = (unsigned)std::min<uint64_t>((n + 4 * kHistThreads - 1) / (4 * kHistThreads),
                                                       (uint64_t)ctx->sm_count * 4);
-  k_sort_hist<<<hgrid, kHistThreads, 0, s>>>(c.in[c.key], n, c.flip, st, plan);
+  k_sort_hist<<<hgrid, kHistThreads, 0, s>>>(c.in[c.key], n, c.flip, st);
   GBJ_TRY(after_launch(ctx, "k_sort_hist", s));
   auto kern = k_sort_pass<kItems, W>;
   GBJ_CHECK_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (int pass = 0; pass < 4; ++pass) {
-    kern<<<ntiles, kThreads, smem, s>>>(c, n, pass, plan, st, buf, buf + n, buf + 2 * (uint64_t)n,
+    kern<<<ntiles, kThreads, smem, s>>>(c, n, pass, st, buf, buf + n, buf + 2 * (uint64_t)n,
                                         buf + 3 * (uint64_t)n, status + pass * words, ctx->d_status);
     GBJ_TRY(after_launch(ctx, "k_sort_pass", s));
   }
@@ -466,7 +460,11 @@ extern "C" int gbj_sort_by_key(gbj_ctx *ctx, const int32_t *const *d_cols, int32
   if (n <= kBlockThreads) return sort_block<1>(ctx, c, (uint32_t)n, s);
   if (n <= 4 * kBlockThreads) return sort_block<4>(ctx, c, (uint32_t)n, s);
   if (n <= kBlockMax) return sort_block<kBlockItems>(ctx, c, (uint32_t)n, s);
-  if (n < (1u << 20)) return sort_tiles<kSmallItems, uint32_t>(ctx, c, (uint32_t)n, s);
+  if (n < (1u << 20)) {
+    const int rc = sort_tiles<kSmallItems, uint32_t>(ctx, c, (uint32_t)n, s);
+    if (rc != GBJ_ERR_OOM) return rc;
+    // a pool without room for the small tiles' status words: a third as many
+  }
   if (n < (1u << 30)) return sort_tiles<kBigItems, uint32_t>(ctx, c, (uint32_t)n, s);
   return sort_tiles<kBigItems, unsigned long long>(ctx, c, (uint32_t)n, s);
 }
