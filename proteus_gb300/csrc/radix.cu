@@ -1164,13 +1164,15 @@ int gbj_partition(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_payload,
 
 }  // extern "C"
 
-// Shared body of gbj_radix_join_agg and gbj_radix_join_agg_minor.
-static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int32_t *d_build_minor,
+// Shared body of gbj_radix_join_agg and gbj_radix_join_agg_minor.  `least`: an
+// untuned call takes the fewest partitions that fit, whose offsets are the
+// fewest words.
+static int radix_join_plan(gbj_ctx *ctx, const int32_t *d_build_keys, const int32_t *d_build_minor,
                            const int32_t *d_build_payload, uint64_t n_build,
                            const int32_t *d_probe_keys, const int32_t *d_probe_minor,
                            const int32_t *d_probe_payload, uint64_t n_probe,
                            const gbj_radix_params *params, const gbj_agg *aggs, int32_t n_aggs,
-                           int64_t *d_out, void *stream) {
+                           int64_t *d_out, void *stream, bool least) {
   if (!ctx || !d_out) return GBJ_ERR_INVALID;
   GBJ_TRY(validate_aggs(ctx, aggs, n_aggs));
   if (n_build >= (1ULL << 31) || n_probe >= (1ULL << 31))
@@ -1232,12 +1234,12 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
       const int b = params->bits > 0 ? params->bits : params->log_parts;
       block = radix_fit_bits(n_build, kJoinPair.rmax) <= b ? kJoinPair.threads : kJoinWide.threads;
     } else {
-      block = radix_auto_threads(n_build, n_probe);
+      block = least ? kJoinPair.threads : radix_auto_threads(n_build, n_probe);
     }
   }
   const JoinShape shape = block == kJoinWide.threads ? kJoinWide : kJoinPair;
   const uint32_t kRMax = (uint32_t)shape.rmax;
-  int bits = radix_auto_bits(n_build, n_probe, shape.threads);
+  int bits = least ? radix_fit_bits(n_build, shape.rmax) : radix_auto_bits(n_build, n_probe, shape.threads);
   if (!explicit_bits) {  // an autotuned choice for this size bucket, if any
     const int32_t tb = tuned_value(ctx, tune_key(shape.threads == kJoinWide.threads ? "radix" : "radix512",
                                                  n_build, n_probe));
@@ -1280,6 +1282,20 @@ static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int3
                                                                  sentinel_part, rc, d_out, ctr, s);
   return launch_join_agg<kJoinPair.rmax, kJoinPair.threads, 2>(ctx, by_rows, spec, R, ro, S, so, items, P, w,
                                                                sentinel_part, rc, d_out, ctr, s);
+}
+
+static int radix_join_impl(gbj_ctx *ctx, const int32_t *d_build_keys, const int32_t *d_build_minor,
+                           const int32_t *d_build_payload, uint64_t n_build,
+                           const int32_t *d_probe_keys, const int32_t *d_probe_minor,
+                           const int32_t *d_probe_payload, uint64_t n_probe,
+                           const gbj_radix_params *params, const gbj_agg *aggs, int32_t n_aggs,
+                           int64_t *d_out, void *stream) {
+  auto plan = [&](bool least) {
+    return radix_join_plan(ctx, d_build_keys, d_build_minor, d_build_payload, n_build, d_probe_keys, d_probe_minor,
+                           d_probe_payload, n_probe, params, aggs, n_aggs, d_out, stream, least);
+  };
+  const int rc = plan(false);
+  return rc == GBJ_ERR_OOM ? plan(true) : rc;  // a pool without room for as many partitions
 }
 
 extern "C" {
