@@ -211,30 +211,85 @@ __device__ __forceinline__ uint32_t hits4(const int4 &k, int32_t kf) {
 }
 __device__ __forceinline__ bool room4(const int4 &k) { return (k.x == 0) | (k.y == 0) | (k.z == 0) | (k.w == 0); }
 
-// A row's slot in a table at `bk` (global or shared memory): it claims the
-// first free slot of its home bucket, starting at a slot chosen by the top
-// hash bits, then of the following buckets.  rows may be null.  False: full.
 __device__ __forceinline__ unsigned long long jb_word(int32_t kf, int32_t value) {
   return ((unsigned long long)(uint32_t)value << 32) | (uint32_t)kf;
 }
-__device__ __forceinline__ bool jb_place(unsigned long long *bk, int32_t *rows, uint32_t bmask, uint32_t h, int32_t kf,
-                                         int32_t value, int32_t row1, bool &dup) {
+// A bucket's empty slots while rows are being placed; dup: one of the others has
+// key kf.
+__device__ __forceinline__ uint32_t jb_empty(const unsigned long long *bucket, int32_t kf, bool &dup) {
+  unsigned long long w[4];
+  asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+               : "l"(bucket)
+               : "memory");
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m |= (uint32_t)(w[i] == 0) << i;
+    dup |= (int32_t)(uint32_t)w[i] == kf;
+  }
+  return m;
+}
+
+// A row's slot in a table at `bk`: it claims the first free slot of its home
+// bucket, starting at a slot chosen by the top hash bits, then of the following
+// buckets; a bucket is passed when it is full.  All lanes call it, `todo` with a
+// row; rows may be null.  False: full.
+//
+// The home slot is claimed unseen, which is all there is to do for most rows;
+// after that a bucket is read before one slot of it is claimed: copies of a key
+// ask for the same slots at the same time, and a claim that fails costs as much
+// as one that does not.  Where a warp has kTogether copies of one key and more,
+// those go on together, one read for all of them and each at another slot.
+// Measured on GB300, build with its clear, us, with a claim for every slot on the
+// way / now: 4 M rows, 1, 2, 3 and 16 a key 139 / 138, 238 / 181, 310 / 207, 1046
+// / 416; 10,000 rows with 16, 2 and 1 keys 792 / 710, 3115 / 1398, 8836 / 2061.
+constexpr int kTogether = 8;
+
+__device__ __forceinline__ bool jb_place(unsigned long long *bk, int32_t *rows, uint32_t bmask, bool todo, uint32_t h,
+                                         int32_t kf, int32_t value, int32_t row1, bool &dup) {
   uint32_t b = h & bmask;
   const uint32_t o = h >> 30;  // start slot (high bits, independent of the bucket for 2^30 buckets or fewer)
-  for (uint32_t step = 0; step <= bmask; ++step) {
-#pragma unroll 1
-    for (uint32_t j = 0; j < 4; ++j) {
-      const uint64_t sl = 4ull * b + ((o + j) & 3u);
-      const unsigned long long old = atomicCAS(&bk[sl], 0ull, jb_word(kf, value));
-      if (old == 0) {
-        if (rows) rows[sl] = row1;
-        return true;
-      }
-      dup |= (int32_t)(uint32_t)old == kf;
+  const unsigned long long word = jb_word(kf, value);
+  auto claim = [&](uint32_t bucket, uint32_t i) {
+    const uint64_t sl = 4ull * bucket + i;
+    const unsigned long long old = atomicCAS(&bk[sl], 0ull, word);
+    if (old == 0) {
+      if (rows) rows[sl] = row1;
+      todo = false;
     }
-    b = (b + 1) & bmask;
+    dup |= (int32_t)(uint32_t)old == kf;  // no row's kf is 0
+  };
+  if (todo) claim(b, o);
+  const int lane = threadIdx.x & 31;
+  // a bucket is looked at again only when another row took a slot meanwhile
+  const uint64_t most = 5ull * (bmask + 1ull);
+  for (;;) {
+    const unsigned left = __ballot_sync(0xffffffffu, todo);
+    if (__popc(left) < kTogether) break;
+    const int32_t lk = __shfl_sync(0xffffffffu, kf, __ffs(left) - 1);
+    uint32_t lb = __shfl_sync(0xffffffffu, b, __ffs(left) - 1);
+    unsigned group = __ballot_sync(0xffffffffu, todo && kf == lk);
+    if (__popc(group) < kTogether) break;
+    for (uint64_t looks = 0; group; ++looks) {
+      if (looks == most) return false;
+      const uint32_t m = jb_empty(bk + 4ull * lb, lk, dup);
+      dup |= __popc(group) > 1;
+      if (todo && kf == lk) {
+        const uint32_t i = __fns(m, 0, __popc(group & ((1u << lane) - 1u)) + 1);
+        if (i < 4) claim(lb, i);
+      }
+      if (__popc(group) >= __popc(m)) lb = (lb + 1) & bmask;
+      group = __ballot_sync(0xffffffffu, todo && kf == lk);
+    }
   }
-  return false;
+  for (uint64_t looks = 0; todo; ++looks) {
+    if (looks == most) return false;
+    const uint32_t m = jb_empty(bk + 4ull * b, kf, dup);
+    if (m) claim(b, (o + __ffs((m | m << 4) >> o) - 1) & 3u);
+    else b = (b + 1) & bmask;
+  }
+  return true;
 }
 
 // meta[0]: a duplicate build key was seen; meta[1]: side-list length.  One
@@ -246,11 +301,14 @@ __global__ void __launch_bounds__(kThreads)
                uint32_t *__restrict__ meta, int32_t *__restrict__ side, uint32_t *status) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   bool dup = false;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int32_t key = keys[i], kf = key ^ kKeyFlip;
-    const int32_t val = payload ? payload[i] : (int32_t)(i + 1);
-    if (kf == 0) side[atomicAdd(&meta[1], 1u)] = (int32_t)i;  // INT32_MIN: the side list
-    else if (!jb_place(bk, rows, bmask, gbjd::fmix32((uint32_t)key), kf, val, (int32_t)(i + 1), dup))
+  const int lane = threadIdx.x & 31;
+  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x - lane; base < n; base += stride) {
+    const uint64_t i = base + lane;
+    const bool in = i < n;
+    const int32_t key = in ? keys[i] : 0, kf = key ^ kKeyFlip;
+    const int32_t val = in && payload ? payload[i] : (int32_t)(i + 1);
+    if (in && kf == 0) side[atomicAdd(&meta[1], 1u)] = (int32_t)i;  // INT32_MIN: the side list
+    if (!jb_place(bk, rows, bmask, in && kf != 0, gbjd::fmix32((uint32_t)key), kf, val, (int32_t)(i + 1), dup))
       gbjd::latch(status, GBJ_DEV_CAPACITY);
   }
   if (dup) meta[0] = 1;
@@ -258,9 +316,12 @@ __global__ void __launch_bounds__(kThreads)
 
 // A small table (at most kSmallSlots slots) in one CTA: built in shared memory
 // and written out whole, so that it needs no clearing before it and no chain
-// of L2 atomics.  Build, start values and 60,000 probes on the GPU, 100, 1000
-// and 4000 rows with payloads: 16.6, 18.6, 25.0 us; cleared and built in L2
-// 20.7, 26.7, 30.8 us.
+// of L2 atomics.  A row takes a slot with one addition to its bucket's count (a
+// claim of each slot by a 64-bit CAS on shared memory made copies of a key wait
+// for one another: 4000 rows with 1, 2 and 16 keys 4260, 6198, 988 us, now 383,
+// 717, 166), and copies are looked for when the table is complete.  Build and
+// clear, 100, 1000 and 4000 unique rows with payloads: 17, 17, 17 us on the host's
+// clock, cleared and built in L2 22, 25, 27.
 constexpr int kSmallThreads = 1024;
 constexpr uint32_t kSmallSlots = 8192;
 
@@ -280,24 +341,59 @@ __global__ void __launch_bounds__(kSmallThreads)
     key[u] = i < n ? __ldg(keys + i) : 0;
     val[u] = payload ? (i < n ? __ldg(payload + i) : 0) : (int32_t)(i + 1);
   }
-  const uint32_t words = slots * (rows ? 12 : 8) / 16;
-  for (uint32_t i = threadIdx.x; i < words; i += kSmallThreads) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
+  const uint32_t nbk = slots / 4, words = slots * (rows ? 12 : 8) / 16;
+  uint32_t *s_fill = reinterpret_cast<uint32_t *>(smem + words * 16);  // rows that asked for the bucket
+  for (uint32_t i = threadIdx.x; i < words + nbk / 4; i += kSmallThreads)
+    reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x < 2) s_meta[threadIdx.x] = 0;
   __syncthreads();
-  bool dup = false;
+  uint32_t at[kPer];  // the row's bucket
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const uint32_t i = threadIdx.x + u * kSmallThreads;
-    if (i >= n) continue;
     const int32_t kf = key[u] ^ kKeyFlip;
-    if (kf == 0) side[atomicAdd(&s_meta[1], 1u)] = (int32_t)i;
-    else jb_place(s_bk, s_rows, slots / 4 - 1, gbjd::fmix32((uint32_t)key[u]), kf, val[u], (int32_t)(i + 1), dup);  // 2 n slots
+    at[u] = gbjd::fmix32((uint32_t)key[u]) & (nbk - 1);
+    if (i >= n) continue;
+    if (kf == 0) {
+      side[atomicAdd(&s_meta[1], 1u)] = (int32_t)i;
+      continue;
+    }
+    for (;;) {  // ends: the table has 2 n slots
+      if (*(volatile uint32_t *)&s_fill[at[u]] < 4) {
+        const uint32_t j = atomicAdd(&s_fill[at[u]], 1u);
+        if (j < 4) {
+          s_bk[4 * at[u] + j] = jb_word(kf, val[u]);
+          if (rows) s_rows[4 * at[u] + j] = (int32_t)(i + 1);
+          break;
+        }
+      }
+      at[u] = (at[u] + 1) & (nbk - 1);
+    }
   }
-  if (dup) s_meta[0] = 1;
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < slots / 2; i += kSmallThreads) bk[i] = reinterpret_cast<const uint4 *>(s_bk)[i];
+  // copies of a key: two in one bucket, or one in a bucket that another passed
+  bool dup = false;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int32_t kf = key[u] ^ kKeyFlip;
+    for (uint32_t b = gbjd::fmix32((uint32_t)key[u]) & (nbk - 1);
+         threadIdx.x + u * kSmallThreads < n && kf != 0 && !dup && b != at[u]; b = (b + 1) & (nbk - 1)) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dup |= (int32_t)(uint32_t)s_bk[4 * b + j] == kf;
+    }
+  }
+  for (uint32_t b = threadIdx.x; b < nbk; b += kSmallThreads) {
+    const uint4 x = reinterpret_cast<const uint4 *>(s_bk)[2 * b], y = reinterpret_cast<const uint4 *>(s_bk)[2 * b + 1];
+    bk[2 * b] = x;
+    bk[2 * b + 1] = y;
+    // {key, value} twice each; 0 is no key
+    dup |= (x.x == x.z && x.x) || (x.x == y.x && x.x) || (x.x == y.z && x.x) || (x.z == y.x && x.z) ||
+           (x.z == y.z && x.z) || (y.x == y.z && y.x);
+  }
   if (rows)
-    for (uint32_t i = threadIdx.x; i < slots / 4; i += kSmallThreads) rows[i] = reinterpret_cast<const uint4 *>(s_rows)[i];
+    for (uint32_t i = threadIdx.x; i < nbk; i += kSmallThreads) rows[i] = reinterpret_cast<const uint4 *>(s_rows)[i];
+  if (__syncthreads_or(dup) && threadIdx.x == 0) s_meta[0] = 1;
+  __syncthreads();
   if (threadIdx.x < 2) meta[threadIdx.x] = s_meta[threadIdx.x];
 }
 
@@ -1248,9 +1344,9 @@ int gbj_join_build(gbj_ctx *ctx, const int32_t *d_keys,
     return code;
   };
   if (n && slots <= kSmallSlots) {
-    const size_t smem = slots * (with_pay ? 12 : 8);
+    const size_t smem = slots * (with_pay ? 13 : 9);
     cudaError_t e = cudaFuncSetAttribute(k_jb_build_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kSmallSlots * 12));
+                                         (int)(kSmallSlots * 13));
     if (e != cudaSuccess) return fail(cuda_error(ctx, e, "k_jb_build_small"));
     k_jb_build_small<<<1, kSmallThreads, smem, s>>>(d_keys, d_payload, (uint32_t)n, static_cast<uint4 *>(mem),
                                                     reinterpret_cast<uint4 *>(t->rows), (uint32_t)slots, t->meta,
