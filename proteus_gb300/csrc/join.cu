@@ -747,7 +747,9 @@ __device__ __forceinline__ JBucket64 ld_bucket64(const JBucket64 *p) {
 // from marked buckets only, where a full bucket used to send every probe of a
 // key that is not unique to the next one (1.5 M rows, two a key, 20 M probes:
 // 541 -> 391 us; unique keys, half of the probes without a match: 224 -> 208;
-// the build, with its clear, takes 85 and 51 us, 74 and 50 without the marks).
+// the build with its clear, without marks / with them: 4 M rows unique 167 / 173,
+// two a key 209 / 218, sixteen 871 / 1033; reading a bucket before its slots are
+// claimed or marked is better for sixteen, 670, and worse for two, 260).
 __global__ void __launch_bounds__(kThreads)
     k_jb64_build(const int64_t *__restrict__ keys, const int32_t *__restrict__ payload, uint64_t n,
                  JBucket64 *__restrict__ bk, uint64_t bmask, uint32_t *__restrict__ meta,
