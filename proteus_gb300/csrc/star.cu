@@ -128,6 +128,10 @@ __device__ __forceinline__ int32_t attr_at(const DimDev &d, int a, uint32_t i) {
                                   : (static_cast<const int32_t *>(d.attr[a]))[i];
 }
 
+// Copies of each query's groups: batches of few queries leave room for them in
+// the array that 64 queries share.
+__host__ __device__ constexpr uint32_t group_copies(int nq) { return (uint32_t)(kMaxQ / nq < 16 ? kMaxQ / nq : 16); }
+
 constexpr int kMaskThreads = 1024;
 constexpr uint32_t kMaskChunk = 8 * kMaskThreads;  // rows of a CTA
 constexpr uint32_t kMaskTable = 4096;              // table entries of a dimension
@@ -297,7 +301,10 @@ struct StarSmem {
 // are neighbours and two lanes add them in one instruction: one L2 operation
 // a match.  Measured on GB300, 64 queries, 2^28 rows: 5.89 ms before, 3.68 ms now
 // (226 warp instructions per 32 rows, 24 active lanes, 3.1 L2 requests a row;
-// the shared and L1 data pipe at 76 %).
+// the shared and L1 data pipe at 76 %).  Where few queries without a filter have
+// few groups, the additions wait for their turn at the groups' sectors; the
+// CTAs then add to different copies of them (2^24 rows, 4 such queries, 35
+// groups each: 5.27 -> 1.27 ms; 64 queries without a filter as before).
 template <bool kVec, bool kKeyed>
 __global__ void __launch_bounds__(kFactThreads, 1)
     k_star_fact(const Desc *__restrict__ desc, FactDev f, Dims dims, StarSmem lay,
@@ -350,6 +357,7 @@ __global__ void __launch_bounds__(kFactThreads, 1)
   }
   __syncthreads();
   const uint64_t active = nq >= 64 ? ~0ull : ((1ull << nq) - 1);
+  const uint32_t copies = group_copies(nq), copy = blockIdx.x % copies;
 
   uint32_t rn = 0, rh = 0;  // the ring's length and head (warp-uniform)
   // the matches of the first c (<= 32) rows of the ring
@@ -377,7 +385,7 @@ __global__ void __launch_bounds__(kFactThreads, 1)
           key[s] = (uint32_t)x - (uint32_t)gs.gmin[s];
         }
         if (key[0] >= gs.gspan[0] || key[1] >= gs.gspan[1]) gbjd::latch(status, GBJ_DEV_INVALID);
-        else gi = (int64_t)q * kMaxGroups + key[0] * gs.gspan[1] + key[1];
+        else gi = ((int64_t)q * copies + copy) * kMaxGroups + key[0] * gs.gspan[1] + key[1];
       }
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -544,13 +552,20 @@ __global__ void __launch_bounds__(kEmitThreads)
   if (q >= desc->nq) return;
   const QDev &qd = desc->q[q];
   const uint32_t ngroups = qd.gspan[0] * qd.gspan[1];
-  const ulonglong2 *acc = reinterpret_cast<const ulonglong2 *>(groups) + (uint64_t)q * kMaxGroups;  // {count, sum}
+  const uint32_t copies = group_copies(desc->nq);
+  const ulonglong2 *acc = reinterpret_cast<const ulonglong2 *>(groups) + (uint64_t)q * copies * kMaxGroups;  // {count, sum}
   const uint32_t g0 = threadIdx.x * 4;
-  unsigned long long c[4];
+  unsigned long long c[4], sum[4];
   uint32_t mine = 0;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    c[u] = g0 + u < ngroups ? acc[g0 + u].x : 0;
+    c[u] = sum[u] = 0;
+    if (g0 + u < ngroups)
+      for (uint32_t k = 0; k < copies; ++k) {
+        const ulonglong2 x = acc[(uint64_t)k * kMaxGroups + g0 + u];
+        c[u] += x.x;
+        sum[u] += x.y;
+      }
     mine += c[u] != 0;
   }
   // exclusive scan of `mine` over the CTA
@@ -586,7 +601,7 @@ __global__ void __launch_bounds__(kEmitThreads)
     qd.out_a[pos] = qd.gmin[0] + (int32_t)(gi / qd.gspan[1]);
     qd.out_b[pos] = qd.gmin[1] + (int32_t)(gi % qd.gspan[1]);
     qd.out_cnt[pos] = (int64_t)c[u];
-    qd.out_sum[pos] = (int64_t)acc[gi].y;
+    qd.out_sum[pos] = (int64_t)sum[u];
     ++pos;
   }
   if (threadIdx.x == 0) *qd.out_n = total;
