@@ -923,7 +923,8 @@ __global__ void __launch_bounds__(kThreads, kCtas)
         bool active = j0 + lane < ns;
         const int2 t = active ? __ldcs(Sp + j0 + lane) : make_int2(0, 0);
         uint32_t hh = __umulhi((uint32_t)t.x, cap);
-        for (uint32_t step = 0; step < cap && __any_sync(0xffffffffu, active); ++step) {
+        for (uint32_t step = 0; step < cap; ++step) {
+          if (!__any_sync(0xffffffffu, active)) break;
           const unsigned short idx = active ? sm.x.tab[hh] : 0;
           active = idx != 0;
           const int2 bt = active ? sm.x.pair[idx - 1] : make_int2(0, 0);
