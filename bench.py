@@ -297,7 +297,8 @@ class PlainJoin:
         return self.ns
 
     def kernel_bytes(self, name):
-        return {"k_jb_probe_agg": 8 * self.ns,   # probe key + payload
+        return {"k_jb_probe_ring": 8 * self.ns,  # probe key + payload
+                "k_jb_probe_agg": 8 * self.ns,
                 "k_jb_build": 12 * self.nr}.get(name)  # key + payload read, bucket slot write
 
     def extra(self, ms, steps, peak):

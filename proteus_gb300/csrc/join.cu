@@ -1196,7 +1196,7 @@ void launch_jb_pairs(int sm_count, const gbj_table *t, uint64_t nbk, const typen
 // Probe kernel over a bucketed table: 16-byte probe loads when both probe
 // columns are aligned, the specialised accumulators, the table's layout.
 template <bool kPay>
-void launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, const int32_t *pay, uint64_t n,
+const char *launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, const int32_t *pay, uint64_t n,
                        const gbj::AggSpec &spec, int64_t *out, cudaStream_t s) {
   const bool vec = ((uintptr_t)keys % 16 == 0) && (!pay || (uintptr_t)pay % 16 == 0);
   const bool two = spec.n == 2 && spec.op[0] == GBJ_AGG_COUNT && spec.op[1] == GBJ_AGG_SUM;
@@ -1206,7 +1206,7 @@ void launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, co
   const uint32_t bmask = (uint32_t)(nbk - 1);
   if (!is_xor && !(two && spec.operand[1] == GBJ_VAL_PRODUCT)) {
     launch_jb_list<JLayout32<kPay>>(sm_count, t, nbk, keys, pay, n, spec, out, s);
-    return;
+    return "k_jb_probe_list";
   }
   const int gv = grid_for_sms(sm_count, (n + kJbGroup - 1) / kJbGroup, kThreads, 2);
   const int gs = grid_for_sms(sm_count, n, kThreads);
@@ -1222,12 +1222,14 @@ void launch_jb_probe_t(int sm_count, const gbj_table *t, const int32_t *keys, co
     else GBJ_JB_PROBE(false, kAggCountProduct);
   }
 #undef GBJ_JB_PROBE
+  return ring ? "k_jb_probe_ring" : "k_jb_probe_agg";
 }
 
-void launch_jb_probe(int sm_count, const gbj_table *t, const int32_t *keys, const int32_t *pay, uint64_t n,
-                     const gbj::AggSpec &spec, int64_t *out, cudaStream_t s) {
-  if (t->rows) launch_jb_probe_t<true>(sm_count, t, keys, pay, n, spec, out, s);
-  else launch_jb_probe_t<false>(sm_count, t, keys, pay, n, spec, out, s);
+// Returns the name of the kernel that it launched.
+const char *launch_jb_probe(int sm_count, const gbj_table *t, const int32_t *keys, const int32_t *pay, uint64_t n,
+                            const gbj::AggSpec &spec, int64_t *out, cudaStream_t s) {
+  if (t->rows) return launch_jb_probe_t<true>(sm_count, t, keys, pay, n, spec, out, s);
+  return launch_jb_probe_t<false>(sm_count, t, keys, pay, n, spec, out, s);
 }
 
 // ------------------------------------------------ allocation-free variant
@@ -1399,8 +1401,8 @@ int gbj_join_probe_agg(gbj_ctx *ctx, const gbj_table *t, const int32_t *d_keys,
   prof_mark(ctx, s);
   GBJ_TRY(init_agg_out(ctx, spec, d_out, s));
   if (n == 0) return GBJ_OK;
-  launch_jb_probe(ctx->sm_count, t, d_keys, d_payload, n, spec, d_out, s);
-  const int rc = after_launch(ctx, "k_jb_probe_agg", s);
+  const char *kernel = launch_jb_probe(ctx->sm_count, t, d_keys, d_payload, n, spec, d_out, s);
+  const int rc = after_launch(ctx, kernel, s);
   note_use(ctx, t->uses, s);
   return rc;
 }
@@ -1421,7 +1423,7 @@ int gbj_join_probe_pairs(gbj_ctx *ctx, const gbj_table *t, const int32_t *d_keys
   const uint64_t nbk = (t->mask + 1) / 4;
   if (t->rows) launch_jb_pairs<JLayout32<true>>(ctx->sm_count, t, nbk, d_keys, d_probe_rows, n, po, s);
   else launch_jb_pairs<JLayout32<false>>(ctx->sm_count, t, nbk, d_keys, d_probe_rows, n, po, s);
-  const int rc = after_launch(ctx, "k_jb_probe_pairs", s);
+  const int rc = after_launch(ctx, "k_jb_probe_list", s);
   note_use(ctx, t->uses, s);
   return rc;
 }
@@ -1516,7 +1518,7 @@ int gbj_join_probe_pairs_i64(gbj_ctx *ctx, const gbj_table *t, const int64_t *d_
   if (n == 0) return GBJ_OK;
   const PairOut po{d_build_rows, d_out_probe_rows, capacity, (unsigned long long *)d_count, ctx->d_status};
   launch_jb_pairs<JLayout64>(ctx->sm_count, t, (t->mask + 1) / 2, d_keys, d_probe_rows, n, po, s);
-  const int rc = after_launch(ctx, "k_jb_probe_pairs", s);
+  const int rc = after_launch(ctx, "k_jb_probe_list", s);
   note_use(ctx, t->uses, s);
   return rc;
 }
