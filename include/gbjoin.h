@@ -78,7 +78,10 @@ int gbj_profile_dump(gbj_ctx *ctx, char *buf, uint64_t buflen);
  * pools (core/platform/lib/memory/memory-manager.cpp,
  * core/platform/lib/memory/buffer-manager.cu).  Allocation is host-side
  * bookkeeping over the block reserved at gbj_ctx_create; nothing calls
- * cudaMalloc after that. */
+ * cudaMalloc after that.  A block may be used on any stream (the call waits
+ * for work that still uses its memory when there is no other); it is given
+ * back behind the context's own stream, so work on other streams that uses it
+ * has to be done when it is freed. */
 int gbj_pool_alloc(gbj_ctx *ctx, uint64_t bytes, void **d_ptr);
 int gbj_pool_free(gbj_ctx *ctx, void *d_ptr);
 int gbj_pool_stats(gbj_ctx *ctx, uint64_t *capacity, uint64_t *in_use,

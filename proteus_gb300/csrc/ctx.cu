@@ -317,7 +317,7 @@ int gbj_profile_dump(gbj_ctx *ctx, char *buf, uint64_t buflen) {
 
 int gbj_pool_alloc(gbj_ctx *ctx, uint64_t bytes, void **d_ptr) {
   if (!ctx || !d_ptr) return GBJ_ERR_INVALID;
-  return pool_alloc(ctx, bytes, ctx->stream, d_ptr);
+  return pool_alloc(ctx, bytes, nullptr, d_ptr);  // for any stream: nothing that one still uses
 }
 
 int gbj_pool_free(gbj_ctx *ctx, void *d_ptr) {

@@ -555,7 +555,7 @@ class Exec {
   template <typename T>
   T *alloc(uint64_t n) {
     void *p = nullptr;
-    ck(gbj_pool_alloc(ctx_, std::max<uint64_t>(n, 1) * sizeof(T), &p), "pool");
+    ck(pool_alloc(ctx_, std::max<uint64_t>(n, 1) * sizeof(T), ctx_->stream, &p), "pool");
     allocs_.push_back(p);
     return static_cast<T *>(p);
   }

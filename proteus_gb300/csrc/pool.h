@@ -32,8 +32,8 @@ struct Pool {
 namespace gbj {
 
 // Takes `size` bytes for work on s: from free ranges and those that s itself
-// gave back, adjacent ones together.  What is left of a range of s stays
-// behind its event.  Waits for other streams' ranges when nothing else fits;
+// gave back, adjacent ones together (s null: for any stream, free ranges only).
+// What is left of a range of s stays behind its event.  Waits for other streams' ranges when nothing else fits;
 // false when that is not enough.
 bool pool_take(Pool &p, uint64_t size, cudaStream_t s, uint64_t *off);
 // Gives [off, off + size) back behind the work enqueued on s so far.

@@ -155,6 +155,17 @@ int main() {
     require(m.take(4, 2) && waits == w + 1, "a third stream did not wait");
     m.check();
   }
+  {  // a block for any stream is nobody's
+    Model m;
+    m.take(kUnits / 2, 0), m.use(0, 0), m.give(0, 0);
+    const int w = waits;
+    uint64_t off;
+    require(gbj::pool_take(m.p, kUnit * kUnits / 2, nullptr, &off) && off == kUnit * kUnits / 2 && waits == w,
+            "a range in use was given to any stream");
+    require(gbj::pool_take(m.p, kUnit, nullptr, &off) && waits == w + 1, "a range in use was not waited for");
+    m.held = {{0, kUnit}, {kUnit * kUnits / 2, kUnit * kUnits / 2}};
+    m.check();
+  }
   for (unsigned seed = 0; seed < 300; ++seed) {
     Model m;
     std::mt19937 rng(seed);
