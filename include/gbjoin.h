@@ -263,7 +263,7 @@ int gbj_radix_join_count_i64(gbj_ctx *ctx, const int64_t *d_r_keys, uint64_t nr,
 /* Every field is honoured or the call fails with GBJ_ERR_UNSUPPORTED: bits
  * and log_parts in [0, 15]; passes 1 needs bits <= 8 and passes 2 bits >= 2
  * (with bits unset, a pinned pass count bounds the automatic choice); block
- * is 0 or the join kernel's 1024 threads. */
+ * is 0, 512 or 1024 (the join kernel's threads). */
 typedef struct gbj_radix_params {
   int32_t bits;       /* radix bits, 0 = autotuned                        */
   int32_t passes;     /* 1 or 2, 0 = one pass up to 12 bits, two above    */
