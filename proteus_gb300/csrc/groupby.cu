@@ -371,13 +371,12 @@ __device__ __forceinline__ void load4(const int32_t *__restrict__ keys, const in
 // either the raw SoA input (items of w rows; level 1 persists across items
 // and is flushed to level 2 when the CTA finishes) or the partitioned AoS
 // pairs (one partition, or a w-row piece of one; level 1 is cleared per
-// item and a whole partition is emitted directly; a partition of up to `one`
-// rows is one item).  kVec: the raw columns are 16-byte aligned and read 4 rows
-// per thread per load.
+// item, and a partition that is one item is emitted directly).  kVec: the raw
+// columns are 16-byte aligned and read 4 rows per thread per load.
 template <bool kPairs, bool kVec>
 __global__ void __launch_bounds__(kThreads, 2)
     k_groupby(const int32_t *__restrict__ keys, const int32_t *__restrict__ vals,
-              const int2 *__restrict__ pairs, uint64_t n, uint64_t w, uint64_t one,
+              const int2 *__restrict__ pairs, uint64_t n, uint64_t w,
               const uint64_t *__restrict__ poff, const uint64_t *__restrict__ item_off, uint32_t P,
               uint32_t tslots, uint32_t rlog, GTable g, Out o, unsigned long long *item_ctr, uint32_t *status) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -408,9 +407,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     bool whole = false;
     if (kPairs) {
       const uint32_t a = gbjd::item_partition(item_off, P, total_items, item);
-      const uint64_t p0 = poff[a], p1 = poff[a + 1];
-      whole = p1 - p0 <= one;
-      lo = p0 + (item - item_off[a]) * w;  // item_off[a] for a whole one
+      const uint64_t p0 = poff[a], p1 = poff[a + 1], i0 = item_off[a];
+      whole = item_off[a + 1] - i0 == 1;
+      lo = p0 + (item - i0) * w;
       hi = whole || lo + w > p1 ? p1 : lo + w;
     } else {
       lo = item * w;
@@ -639,7 +638,7 @@ int groupby_impl(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values, u
     rlog_arg = 0;
     while (rlog_arg < 4 && (size_t)tslots_arg * slot_bytes(rlog_arg + 1) <= kTableBudget) ++rlog_arg;
   };
-  auto launch = [&](auto kern, int tab, const int2 *pairs, uint64_t w, uint64_t one, const uint64_t *poff,
+  auto launch = [&](auto kern, int tab, const int2 *pairs, uint64_t w, const uint64_t *poff,
                     const uint64_t *items, uint32_t P) -> int {
     const size_t smem = (size_t)tab * slot_bytes(rlog_arg);
     // the most any call takes: the limit is the kernel's, not the call's
@@ -647,7 +646,7 @@ int groupby_impl(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values, u
     int per_sm = 1;
     GBJ_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
     per_sm = std::max(per_sm, 1);
-    kern<<<ctx->sm_count * per_sm, kThreads, smem, s>>>(d_keys, d_values, pairs, n, w, one, poff, items,
+    kern<<<ctx->sm_count * per_sm, kThreads, smem, s>>>(d_keys, d_values, pairs, n, w, poff, items,
                                                         P, tslots_arg, rlog_arg, g, o, ctr, ctx->d_status);
     return after_launch(ctx, "k_groupby", s);
   };
@@ -663,8 +662,8 @@ int groupby_impl(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values, u
     tslots_arg = (uint32_t)std::min<uint64_t>(kSlots, std::max<uint64_t>(64, next_pow2(16 * (hint ? hint : groups_cap))));
     pick_rlog();
     const bool aligned = (reinterpret_cast<uintptr_t>(d_keys) | reinterpret_cast<uintptr_t>(d_values)) % 16 == 0;
-    if (aligned) GBJ_TRY(launch(k_groupby<false, true>, (int)tslots_arg, nullptr, wq, 0, nullptr, nullptr, 0));
-    else GBJ_TRY(launch(k_groupby<false, false>, (int)tslots_arg, nullptr, wq, 0, nullptr, nullptr, 0));
+    if (aligned) GBJ_TRY(launch(k_groupby<false, true>, (int)tslots_arg, nullptr, wq, nullptr, nullptr, 0));
+    else GBJ_TRY(launch(k_groupby<false, false>, (int)tslots_arg, nullptr, wq, nullptr, nullptr, 0));
   } else {
     const uint32_t P = 1u << bits;
     pick_rlog();
@@ -677,7 +676,7 @@ int groupby_impl(gbj_ctx *ctx, const int32_t *d_keys, const int32_t *d_values, u
                              nullptr, poff, s));
     k_groupby_plan<<<1, 1024, 0, s>>>(poff, P, w, one, items, ctr);
     GBJ_TRY(after_launch(ctx, "k_groupby_plan", s));
-    GBJ_TRY(launch(k_groupby<true, false>, (int)tslots_arg, pairs, w, one, poff, items, P));
+    GBJ_TRY(launch(k_groupby<true, false>, (int)tslots_arg, pairs, w, poff, items, P));
   }
   const uint64_t emit_threads = 256;
   const uint64_t emit_blocks =
