@@ -401,7 +401,9 @@ __global__ void __launch_bounds__(kFactThreads, 1)
   };
 
   const uint64_t ng = (f.n + 3) / 4, stride = (uint64_t)gridDim.x * kFactThreads;  // groups of four rows
-  for (uint64_t g0 = blockIdx.x * (uint64_t)kFactThreads + (threadIdx.x & ~31u); g0 < ng; g0 += stride) {
+  // (a CTA's warps take groups far apart, so that few rows have all SMs: 10^5
+  // rows, 64 queries without a filter 407 -> 284 us; 2^28 rows unchanged)
+  for (uint64_t g0 = ((threadIdx.x >> 5) * (uint64_t)gridDim.x + blockIdx.x) * 32; g0 < ng; g0 += stride) {
     const uint64_t g = g0 + lane;
     uint32_t k[kMaxDims][4];
     int32_t qty[4], price[4];
