@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 def best_ms(f):
     f()
     best = float("inf")
-    for _ in range(9):
+    for _ in range(25):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record()
         f()
