@@ -11,7 +11,8 @@ namespace gbj {
 // or SoA (out_keys / out_vals).  offsets gets 2^bits + 1 entries.
 // One histogram pass, then one pass per digit group; tuples keep no
 // particular order inside a partition.  passes: 0 = one pass up to 12 bits,
-// two above; 1 = one pass (bits <= 8); 2 = two passes (bits >= 2).
+// two above (two from 9 bits on where the output columns overlap the input);
+// 1 = one pass (bits <= 8); 2 = two passes (bits >= 2).
 // hash_out (GBJ_DIGIT_HASH, AoS output only): each tuple leaves with
 // fmix32(key) in place of the key, as the partitioned join consumes them.
 int partition_tuples(gbj_ctx *ctx, const int32_t *keys, const int32_t *vals,
